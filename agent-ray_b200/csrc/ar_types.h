@@ -2,14 +2,15 @@
 //
 // Wide BVH node (80 bytes, five 16-byte words so one node is five coalesced
 // 128-bit loads): 8 children with 8-bit quantised boxes on a per-node grid.
-//   word0: origin px, py, pz (f32), packed biased exponents ex|ey<<8|ez<<16|imask<<24
-//   word1: child_base, tri_base, meta[0..3], meta[4..7]
+//   word0: origin px, py, pz (f32), packed biased exponents ex|ey<<8|ez<<16
+//   word1: child_base, tri_base, child_mask, tri_mask
 //   word2: qlo_x[0..7], qlo_y[0..7]
 //   word3: qlo_z[0..7], qhi_x[0..7]
 //   word4: qhi_y[0..7], qhi_z[0..7]
-// Child slot s holds: meta[s] == 0 -> empty; imask bit s set -> internal child
-// at child_base + popc(imask & ((1<<s)-1)); otherwise a leaf of
-// (meta[s] >> 5) primitives starting at tri_base + (meta[s] & 31).
+// Child slot s owns bits 4s..4s+3 of the two masks.  child_mask bit 4s: an
+// internal child at child_base + (its rank among the internal children);
+// tri_mask bits 4s..4s+c-1: a leaf of c primitives, the one of mask bit b at
+// tri_base + popc(tri_mask & ((1 << b) - 1)).  Neither: an empty slot.
 // Slots are assigned by octant (bit k of s set: child lies on the + side of
 // axis k), so traversal visits slot (i ^ ray_octant) for i = 0..7, an
 // approximately front-to-back order with no sorting.
@@ -26,9 +27,9 @@ namespace ar {
 
 struct alignas(16) WideNode {
     float px, py, pz;
-    uint32_t exps;  // ex | ey << 8 | ez << 16 | imask << 24
+    uint32_t exps;  // ex | ey << 8 | ez << 16
     uint32_t child_base, tri_base;
-    uint8_t meta[8];
+    uint32_t child_mask, tri_mask;
     uint8_t qlo_x[8], qlo_y[8], qlo_z[8];
     uint8_t qhi_x[8], qhi_y[8], qhi_z[8];
 };

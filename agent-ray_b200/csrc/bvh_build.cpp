@@ -319,22 +319,19 @@ WideBuild build_wide_bvh(const std::vector<PrimBox>& boxes, const BuildOptions& 
         wn.pz = nb.mn[2];
         int e[3];
         for (int k = 0; k < 3; ++k) e[k] = exponent_for(double(nb.mx[k]) - double(nb.mn[k]));
-        uint32_t imask = 0;
         uint32_t n_internal = 0;
         for (int s = 0; s < 8; ++s)
-            if (child_in_slot[s] >= 0 && bn[ch[child_in_slot[s]]].count == 0) { imask |= 1u << s; n_internal++; }
-        wn.exps = uint32_t(e[0] + 127) | uint32_t(e[1] + 127) << 8 | uint32_t(e[2] + 127) << 16 | imask << 24;
+            if (child_in_slot[s] >= 0 && bn[ch[child_in_slot[s]]].count == 0) { wn.child_mask |= 1u << (4 * s); n_internal++; }
+        wn.exps = uint32_t(e[0] + 127) | uint32_t(e[1] + 127) << 8 | uint32_t(e[2] + 127) << 16;
         wn.child_base = uint32_t(out.nodes.size());
         wn.tri_base = uint32_t(out.prim_order.size());
         out.nodes.resize(out.nodes.size() + n_internal);
         uint32_t next_child = wn.child_base;
-        uint32_t tri_off = 0;
         const float p[3] = {wn.px, wn.py, wn.pz};
         for (int s = 0; s < 8; ++s) {
             uint8_t* qlo[3] = {wn.qlo_x, wn.qlo_y, wn.qlo_z};
             uint8_t* qhi[3] = {wn.qhi_x, wn.qhi_y, wn.qhi_z};
             if (child_in_slot[s] < 0) {
-                wn.meta[s] = 0;
                 for (int k = 0; k < 3; ++k) { qlo[k][s] = 255; qhi[k][s] = 0; }
                 continue;
             }
@@ -349,12 +346,10 @@ WideBuild build_wide_bvh(const std::vector<PrimBox>& boxes, const BuildOptions& 
                 qhi[k][s] = uint8_t(hi);
             }
             if (c.count == 0) {
-                wn.meta[s] = 0x80;
                 queue.push_back({ch[child_in_slot[s]], next_child++, it.depth + 1});
             } else {
-                wn.meta[s] = uint8_t((c.count << 5) | tri_off);
+                wn.tri_mask |= ((1u << c.count) - 1u) << (4 * s);
                 for (uint32_t i = 0; i < c.count; ++i) out.prim_order.push_back(order[c.start + i]);
-                tri_off += c.count;
             }
         }
         out.nodes[it.wide] = wn;

@@ -145,13 +145,11 @@ __device__ __forceinline__ TriRecord load_tri(const TriRecord* tris, uint32_t i)
 
 // Per-ray constants of the slab test.
 struct RayPre {
-    f3 o, inv;
+    f3 inv;
     uint32_t oct;  // bit k set when direction k is negative
-    float tmin;
 };
-__device__ __forceinline__ RayPre precompute(f3 o, f3 d, float tmin) {
+__device__ __forceinline__ RayPre precompute(f3 d) {
     RayPre r;
-    r.o = o;
     const float eps = 1e-20f;
     // The reciprocals only cull child boxes, which the builder quantised
     // outward, so the hardware approximation serves (t, u, v and the hit
@@ -164,7 +162,6 @@ __device__ __forceinline__ RayPre precompute(f3 o, f3 d, float tmin) {
     // the octant follows the reciprocal's sign, -0.0 included (its reciprocal
     // is -1e20): near and far planes must swap exactly when inv is negative
     r.oct = (signbit(d.x) ? 1u : 0u) | (signbit(d.y) ? 2u : 0u) | (signbit(d.z) ? 4u : 0u);
-    r.tmin = tmin;
     return r;
 }
 
@@ -214,7 +211,7 @@ constexpr uint32_t kSlotBits = 0x11111111u;
 // Reorders a word of slot flags from slot s to traversal position i = s ^ oct
 // (bytes by one permute, the two slots of a byte by a masked swap).
 __device__ __forceinline__ uint32_t to_traversal_order(uint32_t v, uint32_t oct) {
-    v = __byte_perm(v, 0u, 0x3210u ^ (0x1111u * (oct >> 1)));
+    v = __byte_perm(v, 0u, 0x3210u ^ (0x1111u * ((oct >> 1) & 3u)));
     const uint32_t w = (v ^ (v >> 4)) & ((oct & 1u) * 0x01010101u);
     return v ^ (w * 17u);
 }
@@ -232,24 +229,24 @@ __device__ __forceinline__ uint32_t to_traversal_order(uint32_t v, uint32_t oct)
 // cycles, so instructions are what counts: 16M rays on the 1M-triangle soup
 // 26.4 -> 24.1 ms, extension of a 512x512x16 render of a 139k-triangle scene
 // 6.71 -> 6.37 ms, its shadow rays 4.43 -> 4.13 ms.
-__device__ __forceinline__ uint32_t intersect_node(const WideNode* nodes, uint32_t ni, const RayPre& r, float tmax,
-                                                   uint4& links) {
+__device__ __forceinline__ uint32_t intersect_node(const WideNode* nodes, uint32_t ni, f3 o, f3 inv, uint32_t oct,
+                                                   float tmin, float tmax, uint4& links) {
     const uint4* np = reinterpret_cast<const uint4*>(nodes + ni);
     const uint4 w0 = __ldg(np), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
     links = __ldg(np + 1);
     const float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
     const uint32_t ex = w0.w & 0xffu, ey = (w0.w >> 8) & 0xffu, ez = w0.w >> 16;
-    const float ax = __uint_as_float(ex << 23) * r.inv.x;
-    const float ay = __uint_as_float(ey << 23) * r.inv.y;
-    const float az = __uint_as_float(ez << 23) * r.inv.z;
-    const float bx = (px - r.o.x) * r.inv.x;
-    const float by = (py - r.o.y) * r.inv.y;
-    const float bz = (pz - r.o.z) * r.inv.z;
+    const float ax = __uint_as_float(ex << 23) * inv.x;
+    const float ay = __uint_as_float(ey << 23) * inv.y;
+    const float az = __uint_as_float(ez << 23) * inv.z;
+    const float bx = (px - o.x) * inv.x;
+    const float by = (py - o.y) * inv.y;
+    const float bz = (pz - o.z) * inv.z;
     // pairs: (x, y) of the near and of the far planes, and (near z, far z)
     const uint64_t AXY = f2_pack(ax, ay), BXY = f2_pack(bx, by), AZZ = f2_pack(az, az), BZZ = f2_pack(bz, bz);
     const uint64_t UNBIAS = f2_pack(-8388608.0f, -8388608.0f);
     // near/far plane bytes per axis, chosen by the ray octant
-    const bool nx = r.oct & 1u, ny = r.oct & 2u, nz = r.oct & 4u;
+    const bool nx = oct & 1u, ny = oct & 2u, nz = oct & 4u;
     uint32_t miss = 0;
     const float tfar_limit = tmax * 1.0000004f;
 #pragma unroll
@@ -265,7 +262,7 @@ __device__ __forceinline__ uint32_t intersect_node(const WideNode* nodes, uint32
             f2_unpack(f2_fma(f2_add(f2_pack(biased_byte(nxw, j), biased_byte(nyw, j)), UNBIAS), AXY, BXY), tnx, tny);
             f2_unpack(f2_fma(f2_add(f2_pack(biased_byte(fxw, j), biased_byte(fyw, j)), UNBIAS), AXY, BXY), tfx, tfy);
             f2_unpack(f2_fma(f2_add(f2_pack(biased_byte(nzw, j), biased_byte(fzw, j)), UNBIAS), AZZ, BZZ), tnz, tfz);
-            const float tn = fmax3(tnx, tny, fmaxf(tnz, r.tmin));
+            const float tn = fmax3(tnx, tny, fmaxf(tnz, tmin));
             const float tf = fmin3(tfx, tfy, fminf(tfz, tfar_limit));
             miss = __funnelshift_l(__float_as_uint(tf - tn), miss, 4);
         }
@@ -282,96 +279,120 @@ __device__ __forceinline__ uint32_t intersect_node(const WideNode* nodes, uint32
 // ends the ray.  Kernels drive it with dynamic ray fetch (run_traversal
 // below): a lane whose ray finishes takes the next ray at once, so a warp is
 // not held by its slowest ray.
+//
+// Registers hold only what a node visit and a triangle test read (the current
+// ray, its t limit, the next node, the stack pointer).  What is read once per
+// instance or once per ray lies in named slots below the stack in local
+// memory: the world ray, the best hit so far.  With all of it in scalars the
+// compiler spilled 120-200 bytes inside the node visit, more local traffic
+// than the stack's; now nothing spills at the 64 registers of 8 blocks per SM.
+// 16M rays on the 1M-triangle soup 24.1 -> 20.1 ms, a 139k-triangle scene's
+// extension rays 6.35 -> 5.70 ms and shadow rays 4.11 -> 3.73 ms per
+// 512x512x16 render; 7 blocks (72 registers) 2-12 % slower, 9, 10 and 12
+// blocks (56, 48, 40 registers, spilling again) 2-5, 5-25 and 13-40 %.
 template <bool kAnyHit>
 struct Traverser {
-    static constexpr uint32_t kNodeGroup = 0x80000000u, kMarker = 0x40000000u;
+    static constexpr uint32_t kNodeGroup = 0x80000000u, kMarker = 0x40000000u, kObjectMask = 0x3fffffffu;
+    static constexpr uint32_t kInBlas = 8u;  // in `oct`: the current ray is an instance's local ray
+    // slots of the local array: world origin and t_min, world direction and
+    // t limit (its best hit), world reciprocals and octant, then the best hit
+    // inside the current instance (u, v; slot, scale) and of the ray (u, v;
+    // slot, object); the stack proper starts at kStack
+    static constexpr int kOxy = 0, kOzT = 1, kDxy = 2, kDzT = 3, kIxy = 4, kIzO = 5, kBestUv = 6, kBest = 7, kHitUv = 8,
+                         kHit = 9, kStack = 10;
+    static constexpr int kSlots = kStack + kTraversalStack;
     const DevScene* sc;
-    // World ray: its direction and t_max; its origin and t_min live in wpre
-    // (closest hit, which keeps the world ray's precompute to restore on
-    // instance exit) or in wo/wtmin (any hit, which recomputes it).  Inside an
-    // instance the local ray is pre.o / ld / pre.tmin.
-    f3 wd, wo, ld;
-    float wtmin, wtmax;
-    RayPre pre, wpre;
-    HitRec hit;
-    float ds, best_l, bu, bv;
-    uint32_t cur_inst, best_l_slot, node, guard;
-    uint2 group;
+    f3 o, d, inv;         // the current ray (d is read only inside an instance)
+    float tmin, tlim;     // tlim: the closest hit so far, in the current ray's units
+    uint32_t oct, node, guard;
     int sp;
-    bool in_blas, visit;
 
-    __device__ __forceinline__ void start(const DevScene* s, const Ray& r) {
+    __device__ __forceinline__ static uint2 pk(float a, float b) {
+        return make_uint2(__float_as_uint(a), __float_as_uint(b));
+    }
+    __device__ __forceinline__ void set_ray(f3 no, f3 nd, float nt) {
+        const RayPre r = precompute(nd);
+        o = no;
+        inv = r.inv;
+        oct = r.oct;
+        tmin = nt;
+    }
+
+    // False when the scene is empty (the ray misses).
+    __device__ __forceinline__ bool start(const DevScene* s, const Ray& r, uint2* mem) {
         sc = s;
-        wd = r.d;
-        wtmax = r.tmax;
-        if (kAnyHit) {
-            wo = r.o;
-            wtmin = r.tmin;
-        }
-        hit.t = r.tmax;
-        hit.slot = kInvalid;
-        hit.inst = kInvalid;
-        hit.u = hit.v = 0.f;
-        pre = precompute(r.o, r.d, r.tmin);
-        if (!kAnyHit) wpre = pre;
-        in_blas = false;
-        ds = 1.f;
-        cur_inst = kInvalid;
-        best_l = bu = bv = 0.f;
-        best_l_slot = kInvalid;
-        group = make_uint2(0, 0);
+        set_ray(r.o, r.d, r.tmin);
+        tlim = r.tmax;
+        mem[kOxy] = pk(r.o.x, r.o.y);
+        mem[kOzT] = pk(r.o.z, r.tmin);
+        mem[kDxy] = pk(r.d.x, r.d.y);
+        mem[kDzT] = pk(r.d.z, r.tmax);
+        mem[kIxy] = pk(inv.x, inv.y);
+        mem[kIzO] = make_uint2(__float_as_uint(inv.z), oct);
+        mem[kHit] = make_uint2(kInvalid, kInvalid);
         node = s->tlas_root;
-        visit = node != kInvalid;
         sp = 0;
         guard = 0;
+        return node != kInvalid;
+    }
+
+    // The finished ray's hit (t is the ray's t_max when it missed).
+    __device__ __forceinline__ HitRec result(const uint2* mem) const {
+        HitRec h;
+        h.t = tlim;
+        h.u = h.v = 0.f;
+        h.slot = mem[kHit].x;
+        h.inst = kInvalid;
+        if (!kAnyHit && h.slot != kInvalid) {
+            h.inst = mem[kHit].y;
+            h.u = __uint_as_float(mem[kHitUv].x);
+            h.v = __uint_as_float(mem[kHitUv].y);
+        }
+        return h;
+    }
+
+    __device__ __forceinline__ bool push(uint2 e, int* err, uint2* mem) {
+        if (sp >= kTraversalStack) { atomicExch(err, 1); return false; }
+        mem[kStack + sp++] = e;
+        return true;
     }
 
     // One step = one node visit (with its leaf tests) followed by the stack
     // work that leads to the next node to visit, so every active lane of a
     // warp intersects a node in every step.  Returns true when the ray is
-    // finished (or failed: *err set).  `stack` is the caller's local array
-    // (kept out of the struct so that the scalar state stays in registers).
-    __device__ __forceinline__ bool step(int* err, uint2* stack) {
+    // finished (or failed: *err set).
+    __device__ __forceinline__ bool step(int* err, uint2* mem) {
         if (++guard > (1u << 22)) { atomicExch(err, 3); return true; }
-        if (visit) {
-            uint4 links;  // child_base, tri_base, child_mask, tri_mask
-            const uint32_t met = intersect_node(sc->nodes, node, pre, in_blas ? best_l : (kAnyHit ? wtmax : hit.t), links);
-            group = make_uint2(links.x, to_traversal_order(met & links.z, pre.oct) | (links.z << 1) | kNodeGroup);
-            uint32_t tbits = (met * 15u) & links.w;
-            if (tbits) {
-                if (in_blas) {
-                    while (tbits) {
-                        const uint32_t b = __ffs(tbits) - 1;
-                        tbits &= tbits - 1;
-                        const uint32_t slot = links.y + __popc(links.w & ((1u << b) - 1u));
-                        const TriRecord tr = load_tri(sc->tris, slot);
-                        float t, u, v;
-                        if (tri_test(tr, pre.o, ld, pre.tmin, best_l, t, u, v) && t < best_l) {
-                            if (kAnyHit) {
-                                if (__fdiv_rn(t, ds) < wtmax) {
-                                    hit.t = t;
-                                    hit.slot = slot;
-                                    hit.inst = cur_inst;
-                                    return true;
-                                }
-                            } else {
-                                best_l = t;
-                                best_l_slot = slot;
-                                bu = u;
-                                bv = v;
+        uint4 links;  // child_base, tri_base, child_mask, tri_mask
+        const uint32_t met = intersect_node(sc->nodes, node, o, inv, oct, tmin, tlim, links);
+        uint2 group = make_uint2(links.x, to_traversal_order(met & links.z, oct) | (links.z << 1) | kNodeGroup);
+        uint32_t tbits = (met * 15u) & links.w;
+        if (tbits) {
+            if (oct & kInBlas) {
+                while (tbits) {
+                    const uint32_t b = __ffs(tbits) - 1;
+                    tbits &= tbits - 1;
+                    const uint32_t slot = links.y + __popc(links.w & ((1u << b) - 1u));
+                    const TriRecord tr = load_tri(sc->tris, slot);
+                    float t, u, v;
+                    if (tri_test(tr, o, d, tmin, tlim, t, u, v) && t < tlim) {
+                        if (kAnyHit) {
+                            if (__fdiv_rn(t, __uint_as_float(mem[kBest].y)) < __uint_as_float(mem[kDzT].y)) {
+                                mem[kHit].x = slot;
+                                return true;
                             }
+                        } else {
+                            tlim = t;
+                            mem[kBestUv] = pk(u, v);
+                            mem[kBest].x = slot;
                         }
                     }
-                } else {
-                    // TLAS leaves: resume the node group after the instances.
-                    if (group.y & kSlotBits) {
-                        if (sp >= kTraversalStack) { atomicExch(err, 1); return true; }
-                        stack[sp++] = group;
-                    }
-                    group = make_uint2(0, 0);
-                    if (sp >= kTraversalStack) { atomicExch(err, 1); return true; }
-                    stack[sp++] = make_uint2(links.y, tbits | (links.w << 1));  // leaf group (instances)
                 }
+            } else {
+                // TLAS leaves: resume the node group after the instances.
+                if ((group.y & kSlotBits) && !push(group, err, mem)) return true;
+                group = make_uint2(0, 0);
+                if (!push(make_uint2(links.y, tbits | (links.w << 1)), err, mem)) return true;
             }
         }
         // Find the next node: the nearest child of the current group, else
@@ -380,48 +401,43 @@ struct Traverser {
         for (;;) {
             if (group.y & kSlotBits) {  // a node group with children left (only those stay in `group`)
                 const uint32_t i = __ffs(group.y & kSlotBits) - 1;
-                const uint32_t s = i ^ (4u * pre.oct);
+                const uint32_t s = i ^ (4u * (oct & 7u));
                 node = group.x + __popc(group.y & (kSlotBits << 1) & ((1u << s) - 1u));
                 group.y &= ~(1u << i);
-                if (group.y & kSlotBits) {
-                    if (sp >= kTraversalStack) { atomicExch(err, 1); return true; }
-                    stack[sp++] = group;
-                }
-                group = make_uint2(0, 0);
-                visit = true;
-                return false;
+                return (group.y & kSlotBits) && !push(group, err, mem);
             }
-            if (sp == 0) {
-                visit = false;
-                return true;
-            }
-            const uint2 e = stack[--sp];
+            if (sp == 0) return true;
+            const uint2 e = mem[kStack + --sp];
             if (e.y & kNodeGroup) {
                 group = e;
                 continue;
             }
-            group = make_uint2(0, 0);
             if (e.y & kMarker) {
                 // Leave the instance: convert the local best back to world t.
-                if (!kAnyHit && best_l_slot != kInvalid) {
-                    const float tw = __fdiv_rn(best_l, ds);
-                    if (tw < hit.t) {
-                        hit.t = tw;
-                        hit.slot = best_l_slot;
-                        hit.inst = cur_inst;
-                        hit.u = bu;
-                        hit.v = bv;
+                float best = __uint_as_float(mem[kDzT].y);
+                if (!kAnyHit) {
+                    const uint32_t slot = mem[kBest].x;
+                    if (slot != kInvalid) {
+                        const float tw = __fdiv_rn(tlim, __uint_as_float(e.x));
+                        if (tw < best) {
+                            best = tw;
+                            mem[kHit] = make_uint2(slot, e.y & kObjectMask);
+                            mem[kHitUv] = mem[kBestUv];
+                        }
                     }
                 }
-                in_blas = false;
-                // (any-hit recomputes: keeping the copy costs its kernel more than it saves)
-                pre = kAnyHit ? precompute(wo, wd, wtmin) : wpre;
+                tlim = best;
+                const uint2 a = mem[kOxy], b = mem[kOzT], c = mem[kIxy], f = mem[kIzO];
+                o = mk(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(b.x));
+                tmin = __uint_as_float(b.y);
+                inv = mk(__uint_as_float(c.x), __uint_as_float(c.y), __uint_as_float(f.x));
+                oct = f.y;
                 continue;
             }
             // Instance leaf group: enter the next instance.
             const uint32_t b = __ffs(e.y & kSlotBits) - 1;
             const uint32_t rest = e.y & ~(1u << b);
-            if (rest & kSlotBits) stack[sp++] = make_uint2(e.x, rest);
+            if (rest & kSlotBits) mem[kStack + sp++] = make_uint2(e.x, rest);
             const InstanceRecord* ir = sc->instances + (e.x + __popc(e.y & (kSlotBits << 1) & ((1u << b) - 1u)));
             const float4* ip = reinterpret_cast<const float4*>(ir);
             const float4 m0 = __ldg(ip), m1 = __ldg(ip + 1), m2 = __ldg(ip + 2);
@@ -429,24 +445,25 @@ struct Traverser {
             if (!m3.z) continue;  // mesh without triangles
             const f3 c0 = mk(m0.x, m0.y, m0.z), c1 = mk(m0.w, m1.x, m1.y), c2 = mk(m1.z, m1.w, m2.x),
                      c3 = mk(m2.y, m2.z, m2.w);
+            const uint2 wxy = mem[kDxy], wzt = mem[kDzT];
+            const float wx = __uint_as_float(wxy.x), wy = __uint_as_float(wxy.y), wz = __uint_as_float(wzt.x);
             // glam transform_point3a / transform_vector3a: ((c0*x + c1*y) + c2*z) + c3
-            const f3 w_o = kAnyHit ? wo : wpre.o;
-            const f3 lo = add_rn(c3, add_rn(add_rn(scale_rn(c0, w_o.x), scale_rn(c1, w_o.y)), scale_rn(c2, w_o.z)));
-            const f3 ldu = add_rn(add_rn(scale_rn(c0, wd.x), scale_rn(c1, wd.y)), scale_rn(c2, wd.z));
+            const f3 ldu = add_rn(add_rn(scale_rn(c0, wx), scale_rn(c1, wy)), scale_rn(c2, wz));
             const float scale = __fsqrt_rn(dot_rn(ldu, ldu));
             if (scale < FLT_EPSILON) continue;
-            ds = scale;
-            ld = normalize_rn(ldu);
-            const float ltmin = __fmul_rn(kAnyHit ? wtmin : wpre.tmin, ds);
-            best_l = __fmul_rn(kAnyHit ? wtmax : hit.t, ds);
-            best_l_slot = kInvalid;
-            cur_inst = m3.y;
-            in_blas = true;
-            pre = precompute(lo, ld, ltmin);
-            if (sp >= kTraversalStack) { atomicExch(err, 1); return true; }
-            stack[sp++] = make_uint2(0, kMarker);
+            if (!push(make_uint2(__float_as_uint(scale), kMarker | m3.y), err, mem)) return true;
+            const f3 lo = add_rn(c3, add_rn(add_rn(scale_rn(c0, o.x), scale_rn(c1, o.y)), scale_rn(c2, o.z)));
+            d = normalize_rn(ldu);
+            if (kAnyHit) {
+                mem[kBest].y = __float_as_uint(scale);
+            } else {
+                mem[kBest].x = kInvalid;
+                mem[kDzT].y = __float_as_uint(tlim);
+            }
+            tlim = __fmul_rn(tlim, scale);
+            set_ray(lo, d, __fmul_rn(tmin, scale));
+            oct |= kInBlas;
             node = m3.x;
-            visit = true;
             return false;
         }
     }
@@ -459,7 +476,7 @@ struct Traverser {
 template <bool kAnyHit, class Load, class Store>
 __device__ __forceinline__ void run_traversal(uint32_t* counter, uint32_t n, int* err, Load load, Store store) {
     Traverser<kAnyHit> tr;
-    uint2 stack[kTraversalStack];
+    uint2 mem[Traverser<kAnyHit>::kSlots];
     int cur = -1;
     bool more = true;
     const uint32_t lane = threadIdx.x & 31u;
@@ -477,18 +494,18 @@ __device__ __forceinline__ void run_traversal(uint32_t* counter, uint32_t n, int
                     const DevScene* s;
                     Ray r;
                     load(idx, s, r);
-                    tr.start(s, r);
-                    cur = int(idx);
+                    if (tr.start(s, r, mem)) cur = int(idx);
+                    else store(idx, tr.result(mem));
                 } else {
                     more = false;
                 }
             }
         }
-        if (!__any_sync(0xffffffffu, cur >= 0)) break;
+        if (!__any_sync(0xffffffffu, more || cur >= 0)) break;
         if (cur >= 0) {
             for (int k = 0; k < AR_TRAVERSAL_STEPS; ++k) {
-                if (tr.step(err, stack)) {
-                    store(uint32_t(cur), tr.hit);
+                if (tr.step(err, mem)) {
+                    store(uint32_t(cur), tr.result(mem));
                     cur = -1;
                     break;
                 }

@@ -133,13 +133,13 @@ __device__ __forceinline__ bool tri_test(const TriRecord& tr, f3 o, f3 d, float 
     return true;
 }
 
-__device__ __forceinline__ TriRecord load_tri(const TriRecord* tris, uint32_t i) {
-    const float4* p = reinterpret_cast<const float4*>(tris + i);
+__device__ __forceinline__ TriRecord load_tri(const TriRecord* rec) {
+    const float4* p = reinterpret_cast<const float4*>(rec);
     float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
     TriRecord r;
     r.v0x = a.x; r.v0y = a.y; r.v0z = a.z; r.prim = __float_as_uint(a.w);
     r.e1x = b.x; r.e1y = b.y; r.e1z = b.z; r.object_local = __float_as_uint(b.w);
-    r.e2x = c.x; r.e2y = c.y; r.e2z = c.z; r.pad = __float_as_uint(c.w);
+    r.e2x = c.x; r.e2y = c.y; r.e2z = c.z; r.slot = __float_as_uint(c.w);
     return r;
 }
 
@@ -229,9 +229,9 @@ __device__ __forceinline__ uint32_t to_traversal_order(uint32_t v, uint32_t oct)
 // cycles, so instructions are what counts: 16M rays on the 1M-triangle soup
 // 26.4 -> 24.1 ms, extension of a 512x512x16 render of a 139k-triangle scene
 // 6.71 -> 6.37 ms, its shadow rays 4.43 -> 4.13 ms.
-__device__ __forceinline__ uint32_t intersect_node(const WideNode* nodes, uint32_t ni, f3 o, f3 inv, uint32_t oct,
+__device__ __forceinline__ uint32_t intersect_node(const WideNode* node, f3 o, f3 inv, uint32_t oct,
                                                    float tmin, float tmax, uint4& links) {
-    const uint4* np = reinterpret_cast<const uint4*>(nodes + ni);
+    const uint4* np = reinterpret_cast<const uint4*>(node);
     const uint4 w0 = __ldg(np), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
     links = __ldg(np + 1);
     const float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
@@ -301,7 +301,7 @@ struct Traverser {
     static constexpr int kOxy = 0, kOzT = 1, kDxy = 2, kDzT = 3, kIxy = 4, kIzO = 5, kBestUv = 6, kBest = 7, kHitUv = 8,
                          kHit = 9, kStack = 10;
     static constexpr int kSlots = kStack + kTraversalStack;
-    const DevScene* sc;
+    const WideNode* geom; // the scene's nodes, triangle and instance records
     f3 o, d, inv;         // the current ray (d is read only inside an instance)
     float tmin, tlim;     // tlim: the closest hit so far, in the current ray's units
     uint32_t oct, node, guard;
@@ -320,7 +320,7 @@ struct Traverser {
 
     // False when the scene is empty (the ray misses).
     __device__ __forceinline__ bool start(const DevScene* s, const Ray& r, uint2* mem) {
-        sc = s;
+        geom = s->nodes;
         set_ray(r.o, r.d, r.tmin);
         tlim = r.tmax;
         mem[kOxy] = pk(r.o.x, r.o.y);
@@ -351,6 +351,11 @@ struct Traverser {
         return h;
     }
 
+    // A record's address from its offset in 16-byte words (tri_base, which
+    // for TLAS nodes names instance records).
+    __device__ __forceinline__ const float4* record(uint32_t off) const {
+        return reinterpret_cast<const float4*>(geom) + off;
+    }
     __device__ __forceinline__ bool push(uint2 e, int* err, uint2* mem) {
         if (sp >= kTraversalStack) { atomicExch(err, 1); return false; }
         mem[kStack + sp++] = e;
@@ -364,7 +369,7 @@ struct Traverser {
     __device__ __forceinline__ bool step(int* err, uint2* mem) {
         if (++guard > (1u << 22)) { atomicExch(err, 3); return true; }
         uint4 links;  // child_base, tri_base, child_mask, tri_mask
-        const uint32_t met = intersect_node(sc->nodes, node, o, inv, oct, tmin, tlim, links);
+        const uint32_t met = intersect_node(geom + node, o, inv, oct, tmin, tlim, links);
         uint2 group = make_uint2(links.x, to_traversal_order(met & links.z, oct) | (links.z << 1) | kNodeGroup);
         uint32_t tbits = (met * 15u) & links.w;
         if (tbits) {
@@ -372,19 +377,19 @@ struct Traverser {
                 while (tbits) {
                     const uint32_t b = __ffs(tbits) - 1;
                     tbits &= tbits - 1;
-                    const uint32_t slot = links.y + __popc(links.w & ((1u << b) - 1u));
-                    const TriRecord tr = load_tri(sc->tris, slot);
+                    const TriRecord tr = load_tri(reinterpret_cast<const TriRecord*>(record(links.y)) +
+                                                  __popc(links.w & ((1u << b) - 1u)));
                     float t, u, v;
                     if (tri_test(tr, o, d, tmin, tlim, t, u, v) && t < tlim) {
                         if (kAnyHit) {
                             if (__fdiv_rn(t, __uint_as_float(mem[kBest].y)) < __uint_as_float(mem[kDzT].y)) {
-                                mem[kHit].x = slot;
+                                mem[kHit].x = tr.slot;
                                 return true;
                             }
                         } else {
                             tlim = t;
                             mem[kBestUv] = pk(u, v);
-                            mem[kBest].x = slot;
+                            mem[kBest].x = tr.slot;
                         }
                     }
                 }
@@ -438,8 +443,7 @@ struct Traverser {
             const uint32_t b = __ffs(e.y & kSlotBits) - 1;
             const uint32_t rest = e.y & ~(1u << b);
             if (rest & kSlotBits) mem[kStack + sp++] = make_uint2(e.x, rest);
-            const InstanceRecord* ir = sc->instances + (e.x + __popc(e.y & (kSlotBits << 1) & ((1u << b) - 1u)));
-            const float4* ip = reinterpret_cast<const float4*>(ir);
+            const float4* ip = record(e.x) + 4u * __popc(e.y & (kSlotBits << 1) & ((1u << b) - 1u));
             const float4 m0 = __ldg(ip), m1 = __ldg(ip + 1), m2 = __ldg(ip + 2);
             const uint4 m3 = __ldg(reinterpret_cast<const uint4*>(ip + 3));
             if (!m3.z) continue;  // mesh without triangles

@@ -53,7 +53,7 @@ struct Shade {
 __device__ __forceinline__ Shade make_shade(const DevScene& sc, f3 ro, f3 rd, float t, float u, float v, uint32_t slot,
                                            uint32_t inst) {
     Shade s;
-    const TriRecord tr = load_tri(sc.tris, slot);
+    const TriRecord tr = load_tri(sc.tris + slot);
     const ObjectRecord& ob = sc.objects[inst];
     const MeshRecord mr = sc.meshes[ob.mesh];
     s.prim = tr.prim;

@@ -43,7 +43,7 @@ struct alignas(16) TriRecord {
     float e1x, e1y, e1z;
     uint32_t object_local;  // unused padding
     float e2x, e2y, e2z;
-    uint32_t pad;
+    uint32_t slot;  // this record's index
 };
 static_assert(sizeof(TriRecord) == 48, "triangle record is 48 bytes");
 
@@ -100,9 +100,8 @@ struct alignas(16) LightRecord {
 
 // Read-only view of a device-resident scene, passed by value to kernels.
 struct DevScene {
-    const WideNode* nodes;
-    const TriRecord* tris;
-    const InstanceRecord* instances;  // in TLAS leaf order
+    const WideNode* nodes;  // nodes, triangle and instance records in one buffer
+    const TriRecord* tris;  // the triangle records of that buffer
     const ObjectRecord* objects;
     const MeshRecord* meshes;
     const uint32_t* indices;
@@ -119,7 +118,7 @@ struct DevScene {
     uint32_t tlas_root;       // 0xFFFFFFFF: empty scene
     uint32_t num_lights;
     uint32_t light_dist;      // ar_light_distribution
-    uint32_t num_instances;
+    uint32_t pad;
 };
 
 constexpr uint32_t kInvalid = 0xFFFFFFFFu;

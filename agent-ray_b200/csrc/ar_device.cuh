@@ -64,7 +64,7 @@ __device__ __forceinline__ f3 cross_rn(f3 a, f3 b) {
 }
 // glam normalize: v * (1 / sqrt(dot(v, v)))
 __device__ __forceinline__ f3 normalize_rn(f3 a) {
-    return scale_rn(a, __fdiv_rn(1.0f, __fsqrt_rn(dot_rn(a, a))));
+    return scale_rn(a, __frcp_rn(__fsqrt_rn(dot_rn(a, a))));
 }
 __device__ __forceinline__ f3 ld3(const float* p) { return {p[0], p[1], p[2]}; }
 
@@ -118,7 +118,7 @@ __device__ __forceinline__ bool tri_test(const TriRecord& tr, f3 o, f3 d, float 
     f3 h = cross_rn(d, e2);
     float a = dot_rn(e1, h);
     if (fabsf(a) < 1e-8f) return false;
-    float f = __fdiv_rn(1.0f, a);
+    float f = __frcp_rn(a);
     f3 s = sub_rn(o, v0);
     float uu = __fmul_rn(f, dot_rn(s, h));
     if (uu < 0.0f || uu > 1.0f) return false;
@@ -148,17 +148,27 @@ struct RayPre {
     f3 inv;
     uint32_t oct;  // bit k set when direction k is negative
 };
+// Slab reciprocal: the hardware approximation, +-1e20 at most (a zero keeps its
+// sign).  It only culls child boxes, which the builder quantised outward; t, u,
+// v and the hit itself come from the exactly rounded triangle test.  One
+// approximation and two clamps an axis instead of a test, a select and a
+// division; with __frcp_rn for the exact reciprocals (1/a of the triangle test,
+// 1/length of the local direction: the same correctly rounded value as the
+// division in about half its instructions) 1M visibility rays 451 -> 441 us, a
+// 139k-triangle scene at 512x512x16 11.0 -> 10.8 ms, BDPT room 57.5 -> 56.6 ms.
+__device__ __forceinline__ float slab_rcp(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return fminf(fmaxf(r, -1e20f), 1e20f);
+}
 __device__ __forceinline__ RayPre precompute(f3 d) {
     RayPre r;
-    const float eps = 1e-20f;
     // The reciprocals only cull child boxes, which the builder quantised
     // outward, so the hardware approximation serves (t, u, v and the hit
     // itself come from the exactly rounded triangle test); every parity test
     // gives the same hits, and ray setup and instance entry get cheaper
     // (measured +0.9% closest hit on the soup, +2.4% PT, +1.6% BDPT).
-    r.inv.x = __fdividef(1.0f, fabsf(d.x) > eps ? d.x : copysignf(eps, d.x));
-    r.inv.y = __fdividef(1.0f, fabsf(d.y) > eps ? d.y : copysignf(eps, d.y));
-    r.inv.z = __fdividef(1.0f, fabsf(d.z) > eps ? d.z : copysignf(eps, d.z));
+    r.inv = mk(slab_rcp(d.x), slab_rcp(d.y), slab_rcp(d.z));
     // the octant follows the reciprocal's sign, -0.0 included (its reciprocal
     // is -1e20): near and far planes must swap exactly when inv is negative
     r.oct = (signbit(d.x) ? 1u : 0u) | (signbit(d.y) ? 2u : 0u) | (signbit(d.z) ? 4u : 0u);

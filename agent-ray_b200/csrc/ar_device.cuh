@@ -165,11 +165,6 @@ __device__ __forceinline__ float slab_rcp(float x) {
 }
 __device__ __forceinline__ RayPre precompute(f3 d) {
     RayPre r;
-    // The reciprocals only cull child boxes, which the builder quantised
-    // outward, so the hardware approximation serves (t, u, v and the hit
-    // itself come from the exactly rounded triangle test); every parity test
-    // gives the same hits, and ray setup and instance entry get cheaper
-    // (measured +0.9% closest hit on the soup, +2.4% PT, +1.6% BDPT).
     r.inv = mk(slab_rcp(d.x), slab_rcp(d.y), slab_rcp(d.z));
     // the octant follows the reciprocal's sign, -0.0 included (its reciprocal
     // is -1e20): near and far planes must swap exactly when inv is negative
@@ -177,7 +172,6 @@ __device__ __forceinline__ RayPre precompute(f3 d) {
     return r;
 }
 
-__device__ __forceinline__ uint32_t byte_of(uint32_t w, uint32_t i) { return (w >> (8 * i)) & 0xffu; }
 // Packed pairs of f32 (Blackwell's f32x2 arithmetic: one instruction per
 // pair, each half rounded exactly as the scalar instruction would).
 __device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
@@ -494,8 +488,16 @@ __device__ __forceinline__ void run_traversal(uint32_t* counter, uint32_t n, int
     Traverser<kAnyHit> tr;
     uint2 mem[Traverser<kAnyHit>::kSlots];
     int cur = -1;
-    bool more = true;
     const uint32_t lane = threadIdx.x & 31u;
+    // A warp runs every path that any of its rays needs, so few rays are spread
+    // over the grid's warps, about 1.5 lanes' worth of each warp's share taking
+    // part.  The line lies at 5 rays a warp (kernel time, closest / any hit in an
+    // instanced room, packed against spread: 64 rays 58 / 47 -> 34 / 27 us, 4096
+    // rays 76 / 83 -> 51 / 67, 20000 rays 85 / 84 -> 78 / 80, 40000 rays 95 / 88
+    // -> 93 / 96, 80000 rays 103 / 97 -> 112 / 106: from there on the schedulers
+    // have no free issue slots left).
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    bool more = lane < (n < 5u * warps ? (n + n / 2u + warps - 1u) / warps : 32u);
     for (;;) {
         const bool need = more && cur < 0;
         const uint32_t mask = __ballot_sync(0xffffffffu, need);

@@ -13,7 +13,9 @@
 //   shadow                any hit; visible NEE contributions; finished paths
 //                         deposit into their job's film
 //
-// The tick is captured once per buffer parity as a CUDA graph and replayed.
+// The tick is captured once per buffer parity as a CUDA graph and replayed; a
+// tick's shadow stage runs in the next tick's graph, on a branch beside plan,
+// generate and extend.
 #pragma once
 #include <utility>
 #include <vector>

@@ -1,0 +1,62 @@
+"""Scheduling edges of the traversal and of the path engine: ray counts around
+the line below which rays are spread over the grid's warps, and renders whose
+paths all start in the first tick against renders refilled from a small pool.
+Both must give what any other split of the same work gives."""
+import numpy as np
+import pytest
+
+import agentray
+import agentray.scenes as S
+from agentray import _abi as A
+
+pytestmark = pytest.mark.gpu
+
+
+def test_ray_counts_around_the_spreading_line(ctx):
+    # Every prefix of a batch gives the batch's own hits, bit for bit: one ray,
+    # part of a warp, the largest spread batch and the smallest packed one
+    # (5 rays a warp of the persistent grid), and one above it.
+    import torch
+    sc, _ = S.room(seed=4, sphere_levels=(3, 3, 2, 2), n_boxes=60)
+    g = agentray.Scene(ctx, sc)
+    warps = torch.cuda.get_device_properties(0).multi_processor_count * 8 * 4
+    n = 5 * warps + 1
+    rng = np.random.default_rng(3)
+    ot = np.zeros((n, 4), np.float32)
+    dt = np.zeros((n, 4), np.float32)
+    ot[:, :3] = rng.uniform((0.1, 0.1, 0.1), (9.9, 4.9, 9.9), (n, 3))
+    ot[:, 3] = 1e-4
+    d = rng.normal(size=(n, 3))
+    dt[:, :3] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    dt[:, 3] = 4.0
+    hits, inst = g.trace_closest(ot, dt)
+    occ = g.trace_any(ot, dt)
+    assert 0.05 < occ.mean() < 0.95
+    np.testing.assert_array_equal(occ != 0, inst != 0xFFFFFFFF)
+    for k in (1, 3, 31, 33, 4097, warps, n - 2, n - 1):
+        h, i = g.trace_closest(ot[:k], dt[:k])
+        np.testing.assert_array_equal(h.view(np.uint32), hits[:k].view(np.uint32))
+        np.testing.assert_array_equal(i, inst[:k])
+        np.testing.assert_array_equal(g.trace_any(ot[:k], dt[:k]), occ[:k])
+
+
+@pytest.mark.parametrize("depth", [0, 1, 2, 7])
+def test_render_does_not_depend_on_the_path_pool(depth):
+    # 40x30x4 = 4800 samples: one tick's worth in the default pool (the render
+    # then ends after depth + 1 ticks), refilled over several ticks in a pool of
+    # 4096.  FP64 films: only the order of the additions differs.
+    sc, cam = S.cornell_box(1)
+    images = []
+    for capacity in (1 << 22, 4096):
+        ctx = agentray.Context(0)
+        ctx.set_tuning(path_capacity=capacity)
+        g = agentray.Scene(ctx, sc)
+        pt = agentray.PathTracer(agentray.PathTracerConfig(spp=4, max_depth=depth, rr_depth=3, seed=5,
+                                                           film_precision=A.FILM_F64))
+        images.append([pt.render(g, cam, 40, 30).rgb.copy() for _ in range(3)])
+        g.close()
+        ctx.close()
+    assert images[0][0].max() > 0
+    for pair in images:
+        for img in pair:
+            np.testing.assert_allclose(img, images[0][0], rtol=1e-6, atol=1e-9)

@@ -53,10 +53,6 @@ struct BdParams {
     float4* vb;  // n.xyz, pdf_rev
     float4* vc;  // thr.xyz, info (type << 30 | delta << 29 | index)
     float2* vuv; // tex_uv of surface vertices
-    float4* sva; // the vertex arrays permuted into the (S, T)-sorted sample
-    float4* svb; // order, so the connection kernel's warps read them coalesced
-    float4* svc;
-    float2* svuv;
     uint8_t* nv; // [sub * cap + si]
     float4* thr; // per subpath, at sub * cap + si: thr.xyz, previous directional pdf
     uint32_t* dim;
@@ -96,7 +92,7 @@ struct Vtx {
 __device__ __forceinline__ Vtx load_vtx(const BdParams& P, uint32_t sub, uint32_t k, uint32_t si) {
     const size_t i = vidx(P, sub, k, si);
     // read-only where this is called (connection and MIS stages): through the
-    // non-coherent path (connection stage -2.5%)
+    // non-coherent path
     const float4 a = __ldg(P.va + i), b = __ldg(P.vb + i), c = __ldg(P.vc + i);
     Vtx v;
     v.p = mk(a.x, a.y, a.z);
@@ -133,7 +129,7 @@ __device__ __forceinline__ MatView vtx_mat(const BdParams& P, const BdJob& J, co
     return load_mat_at(J.sc, v.index, uv.x, uv.y);
 }
 
-// pdf_solid_angle_to_area (:305-314) and geometry_term (:318-328)
+// pdf_solid_angle_to_area (:305-314)
 __device__ __forceinline__ float pdf_sa_to_area(float pdf, f3 from, f3 to, f3 n_to) {
     const f3 d = to - from;
     const float d2 = dot(d, d);
@@ -141,14 +137,6 @@ __device__ __forceinline__ float pdf_sa_to_area(float pdf, f3 from, f3 to, f3 n_
     const f3 dir = d / sqrtf(d2);
     return pdf * fabsf(dot(n_to, dir)) / d2;
 }
-__device__ __forceinline__ float geometry_term(f3 pa, f3 na, f3 pb, f3 nb) {
-    const f3 d = pb - pa;
-    const float d2 = dot(d, d);
-    if (d2 < 1e-12f) return 0.f;
-    const f3 dir = d / sqrtf(d2);
-    return fabsf(dot(na, dir)) * fabsf(dot(nb, -dir)) / d2;
-}
-
 __device__ __forceinline__ f3 uniform_sphere(float ux, float uy) {
     const float ct = 1.0f - 2.0f * ux;
     const float st = sqrtf(fmaxf(1.0f - ct * ct, 0.0f));
@@ -217,62 +205,13 @@ __device__ __noinline__ float mis_weight(const BdParams& P, const BdJob& J, uint
 }
 
 // Prefix form of the reference ratio walk for the power heuristic with
-// beta = 2 and no delta surface vertex (the only BSDFs here are Lambertian and
-// GGX).  With q_i = pdf_rev(z_i) / pdf_fwd(z_i) the camera-side terms of
+// beta = 2 and no delta surface vertex (the BSDFs here are Lambertian, GGX and
+// rough glass).  With q_i = pdf_rev(z_i) / pdf_fwd(z_i) the camera-side terms of
 // strategy (s, t) are r1^2 (1 + q_{s-1}^2 + (q_{s-1} q_{s-2})^2 + ...), where
 // r1 = pdf_connect_cam / pdf_fwd(z_{s-1}); the bracket C_s obeys C_1 = 1,
 // C_s = 1 + q_{s-1}^2 C_{s-1}.  The light side is symmetric (D_t), and its
 // t = 1 term counts only for area lights.  Same sums as mis_weight, in FP64.
 constexpr uint32_t kMisCache = 16;
-struct MisCache {
-    double C[kMisCache], D[kMisCache];
-    float fwd_cam[kMisCache], fwd_light[kMisCache];
-    bool fast;
-};
-
-__device__ void build_mis_cache(const BdParams& P, const BdJob& J, uint32_t si, uint32_t S, uint32_t T, MisCache& mc) {
-    mc.fast = J.mis_mode == AR_MIS_POWER && J.mis_beta == 2.0f && S <= kMisCache && T <= kMisCache;
-    if (!mc.fast) return;
-    double c = 1.0;
-    for (uint32_t s = 1; s <= S; ++s) {
-        const Vtx v = load_vtx(P, 0, s - 1, si);
-        if (v.type == kTypeSurface && v.delta) mc.fast = false;
-        mc.fwd_cam[s - 1] = v.pdf_fwd;
-        if (s >= 2) {
-            const double q = double(fmaxf(v.pdf_rev, 0.f)) / double(fmaxf(v.pdf_fwd, 1e-30f));
-            c = 1.0 + q * q * c;
-        }
-        mc.C[s - 1] = c;  // C_s (s >= 1) with q_{s-1} taken from z[s-1]
-    }
-    double d = 1.0;
-    for (uint32_t t = 1; t <= T; ++t) {
-        const Vtx v = load_vtx(P, 1, t - 1, si);
-        if (v.type == kTypeSurface && v.delta) mc.fast = false;
-        mc.fwd_light[t - 1] = v.pdf_fwd;
-        if (t >= 2) {
-            const double q = double(fmaxf(v.pdf_rev, 0.f)) / double(fmaxf(v.pdf_fwd, 1e-30f));
-            d = 1.0 + q * q * d;
-        }
-        mc.D[t - 1] = d;
-    }
-}
-
-__device__ __forceinline__ float mis_weight_cached(const BdParams& P, const BdJob& J, const MisCache& mc, uint32_t si,
-                                                   uint32_t S, uint32_t T, uint32_t s, uint32_t t, float pdf_cc,
-                                                   float pdf_cl, bool light_is_point) {
-    if (!mc.fast) return mis_weight(P, J, si, S, T, s, t, pdf_cc, pdf_cl);
-    if (s + t == 2) return 1.0f;
-    double sum = 0.0;
-    if (s >= 2) {
-        const double r = double(pdf_cc) / double(fmaxf(mc.fwd_cam[s - 1], 1e-30f));
-        sum += r * r * mc.C[s - 1];
-    }
-    if (t >= 2 || (t == 1 && !light_is_point)) {
-        const double r = double(pdf_cl) / double(fmaxf(mc.fwd_light[t - 1], 1e-30f));
-        sum += r * r * mc.D[t - 1];
-    }
-    return float(1.0 / (1.0 + sum));
-}
 
 __device__ __forceinline__ void film_add(const BdJob& J, uint32_t pix, f3 v) {
     if (J.film64) {
@@ -480,120 +419,256 @@ __global__ void __launch_bounds__(256, 4) k_bd_vertex(BdParams P, uint32_t depth
     }
 }
 
-// Out-of-line BSDF bodies for the connection kernel: its warps diverge
-// across strategies, and one copy of each body keeps the instruction
-// footprint small.  Same arithmetic as the inline forms.
-__device__ __noinline__ f3 bsdf_eval_ool(const MatView& m, f3 wi, f3 wo) { return bsdf_eval(m, wi, wo); }
-__device__ __noinline__ float bsdf_pdf_ool(const MatView& m, f3 wi, f3 wo) { return bsdf_pdf(m, wi, wo); }
+// ---- connection stage ----
+// What bounds it is the number of correctly rounded divisions and roots (each a
+// dozen instructions and a branch), the divergence of materials and strategies
+// in a warp, and the latency of its loads at two dozen warps per SM.  A thread
+// per sample that walked all its strategies rebuilt the light vertex's frame and
+// material for every camera vertex, ran in 128 registers, and needed the
+// vertices copied into sorted order first.
+//
+// A block connects a tile of samples (neighbours in the (S, T)-sorted order)
+// that it holds in shared memory: per vertex the record the strategies read,
+// with the shading frame, the local direction toward the previous vertex and
+// the material already worked out, and the MIS prefix sums.  Threads are
+// (strategy, sample): tile_samples consecutive threads take the same strategy
+// (s, t) of the tile's samples.  4.2M samples of the 195k-triangle room at depth
+// 10: sorted copies 2.4 + connection 14.2 -> 8.4 ms, 65k samples of a small scene
+// at depth 8: 310 -> 138 us.  Other shapes (threads x samples, blocks per SM, room
+// / small): 256x32, 2: 8.7 / 152; 512x32, 2: 9.3 / 157; 256x16, 3: 9.0 / 153;
+// 128x16, 5: 9.3 / 139; 64x8, 11: 11.7 / 188; 32x4, 22: 20.7 / 215.  Listing the
+// candidates that a hemisphere test keeps and evaluating them 32 at a time, as
+// whole warps of mixed strategies, was slower (20.3 / 333).
+enum TileField : uint32_t {
+    kFp = 0,      // position
+    kFsmith = 3,  // conductor: sqrt(cos^2 + alpha^2 sin^2) of the direction below
+    kFn = 4,      // stored normal
+    kFinfo = 7,   // type << 30 | material kind << 28 | material or light index
+    kFthr = 8,    // throughput
+    kFalpha = 11,
+    kFon = 12,    // frame: normal
+    kFob = 15,    // frame: bitangent (the tangent is their cross product)
+    kFwo = 18,    // direction toward the previous vertex, in the frame
+    kFcol = 21,   // albedo or f0; a dielectric's eta first
+    kTileFields = 24
+};
+constexpr uint32_t kConnectThreads = 384, kConnectBlocks = 2;  // blocks per SM
+constexpr uint32_t kTileInts = 6;  // per sample: S, T, job, pixel, sample, flags
+
+// Bytes of shared memory of a tile: per sample 2 maxv vertices of 24 floats,
+// a prefix sum and 1 / pdf_fwd^2 (f64), and the sample's integers.
+constexpr size_t tile_bytes(uint32_t maxv, uint32_t samples) {
+    return size_t(samples) * (2 * size_t(maxv) * (kTileFields * 4 + 16) + kTileInts * 4);
+}
+// Samples of a tile: as many as let two blocks share an SM's 227 KB: 32 up to
+// depth 10, 16 up to 21, 8 up to 43, 4 up to 62.
+constexpr size_t kTileMax = 80000;
+constexpr uint32_t tile_samples(uint32_t maxv) {
+    uint32_t n = 32;
+    while (n > 4 && tile_bytes(maxv, n) > kTileMax) n >>= 1;
+    return n;
+}
+static_assert(tile_bytes(63, 4) <= kTileMax && kConnectThreads % 32 == 0, "every depth has a tile");
+
+struct Tile {
+    double* pre;  // [vertex][sample]: C_s, D_t
+    double* inv;  // [vertex][sample]: 1 / pdf_fwd^2
+    float* f;     // [vertex][field][sample]
+    uint32_t* i;  // [int][sample]
+    uint32_t maxv, samples, lane;  // lane: this thread's sample
+    __device__ __forceinline__ uint32_t vertex(uint32_t sub, uint32_t k) const { return sub * maxv + k; }
+    __device__ __forceinline__ float& at(uint32_t v, uint32_t field) const {
+        return f[(v * kTileFields + field) * samples + lane];
+    }
+    __device__ __forceinline__ f3 vec(uint32_t v, uint32_t field) const {
+        return mk(at(v, field), at(v, field + 1), at(v, field + 2));
+    }
+    __device__ __forceinline__ void put(uint32_t v, uint32_t field, f3 x) const {
+        at(v, field) = x.x;
+        at(v, field + 1) = x.y;
+        at(v, field + 2) = x.z;
+    }
+    __device__ __forceinline__ double& prefix(uint32_t v) const { return pre[v * samples + lane]; }
+    __device__ __forceinline__ double& inv_fwd2(uint32_t v) const { return inv[v * samples + lane]; }
+    __device__ __forceinline__ uint32_t& word(uint32_t k) const { return i[k * samples + lane]; }
+    __device__ __forceinline__ Onb frame(uint32_t v) const {
+        Onb o;
+        o.n = vec(v, kFon);
+        o.b = vec(v, kFob);
+        o.t = cross(o.b, o.n);
+        return o;
+    }
+};
+enum TileInt : uint32_t { kIs, kIt, kIjob, kIpix, kIsample, kIflags };
+constexpr uint32_t kFlagFastMis = 1u, kFlagPointLight = 2u;
+
+// BSDF value and density of a tile vertex toward `wi_world`.  The conductor's
+// masking and shadowing takes the form
+//   D G2 / (4 ci co) = D / (2 (co S(wi) + ci S(wo))),  S(w) = sqrt(c^2 + a^2 (1 - c^2)),
+// equal to ggx_lambda's (1 + L(wi) + L(wo)) with S / c = 1 + 2 L, which needs
+// one root and one division where that form takes two roots and four divisions.
+__device__ __noinline__ float4 glass_eval_pdf(float eta, float alpha, f3 wi, f3 wo) {
+    MatView m{};
+    m.kind = AR_MATERIAL_DIELECTRIC;
+    m.alpha = alpha;
+    m.eta = eta;
+    const f3 f = dielectric_eval(m, wi, wo);
+    return make_float4(f.x, f.y, f.z, dielectric_pdf(m, wi, wo));
+}
+__device__ __forceinline__ float smith_root(float alpha, float cos_w) {
+    const float c2 = cos_w * cos_w;
+    return sqrtf(c2 + (alpha * alpha) * (1.0f - c2));
+}
+__device__ __forceinline__ float4 tile_bsdf(const Tile& tl, uint32_t v, f3 wi_world) {
+    const uint32_t kind = (__float_as_uint(tl.at(v, kFinfo)) >> 28) & 3u;
+    const f3 wi = to_local(tl.frame(v), wi_world), wo = tl.vec(v, kFwo), col = tl.vec(v, kFcol);
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (kind == AR_MATERIAL_DIELECTRIC) return glass_eval_pdf(col.x, tl.at(v, kFalpha), wi, wo);
+    if (!same_hemi(wi, wo)) return none;
+    const float ci = fabsf(wi.z), co = fabsf(wo.z);
+    if (kind == AR_MATERIAL_LAMBERTIAN)
+        return make_float4(col.x * kInvPi, col.y * kInvPi, col.z * kInvPi, ci * kInvPi);
+    const f3 hs = wi + wo;
+    const f3 h = hs * __frsqrt_rn(dot(hs, hs));
+    const float whwi = fabsf(dot(wi, h));
+    const float c = fminf(fmaxf(1.0f - whwi, 0.0f), 1.0f), c2 = c * c, c5 = c * (c2 * c2);
+    const float alpha = tl.at(v, kFalpha), a2 = alpha * alpha;
+    const float den = (h.z * h.z) * (a2 - 1.0f) + 1.0f;
+    const float pd = (kPi * den) * den;  // D = a2 / pd
+    const float g = a2 / (pd * (2.0f * (co * smith_root(alpha, ci) + ci * tl.at(v, kFsmith))));
+    const float pdf = whwi == 0.f ? 0.f : (a2 * fabsf(h.z)) / (pd * (4.0f * whwi));
+    return make_float4((col.x + (1.0f - col.x) * c5) * g, (col.y + (1.0f - col.y) * c5) * g,
+                       (col.z + (1.0f - col.z) * c5) * g, pdf);
+}
+
+__device__ __forceinline__ float tile_mis(const BdParams& P, const BdJob& J, const Tile& tl, uint32_t s, uint32_t t,
+                                          float pdf_cc, float pdf_cl) {
+    const uint32_t flags = tl.word(kIflags);
+    if (!(flags & kFlagFastMis))
+        return mis_weight(P, J, tl.word(kIsample), tl.word(kIs), tl.word(kIt), s, t, pdf_cc, pdf_cl);
+    if (s + t == 2) return 1.0f;
+    double sum = 0.0;
+    if (s >= 2) {
+        const uint32_t v = tl.vertex(0, s - 1);
+        sum += (double(pdf_cc) * double(pdf_cc)) * (tl.inv_fwd2(v) * tl.prefix(v));
+    }
+    if (t >= 2 || (t == 1 && !(flags & kFlagPointLight))) {
+        const uint32_t v = tl.vertex(1, t - 1);
+        sum += (double(pdf_cl) * double(pdf_cl)) * (tl.inv_fwd2(v) * tl.prefix(v));
+    }
+    return float(__drcp_rn(1.0 + sum));
+}
+
+// Vertex k of subpath `sub` of the tile's sample: its record, frame and
+// material into shared memory, q^2 of the MIS prefix sums into `pre`.
+__device__ __forceinline__ void tile_load(const BdParams& P, const BdJob& J, const Tile& tl, uint32_t sub, uint32_t k,
+                                          uint32_t si) {
+    const Vtx v = load_vtx(P, sub, k, si);
+    const uint32_t w = tl.vertex(sub, k);
+    tl.put(w, kFp, v.p);
+    tl.put(w, kFn, v.n);
+    tl.put(w, kFthr, v.thr);
+    uint32_t info = (v.type << 30) | v.index;
+    const double fwd = double(fmaxf(v.pdf_fwd, 1e-30f)), rev = double(fmaxf(v.pdf_rev, 0.f));
+    const double inv = __drcp_rn(fwd * fwd);
+    tl.inv_fwd2(w) = inv;
+    tl.prefix(w) = (rev * rev) * inv;
+    if (v.type == kTypeSurface) {
+        const float4 a = __ldg(P.va + vidx(P, sub, k - 1, si));
+        const MatView m = vtx_mat(P, J, v, sub, k, si);
+        // the frame of onb_from_normal
+        Onb o;
+        o.n = v.n * __frsqrt_rn(dot(v.n, v.n));
+        const f3 b = cross(o.n, fabsf(o.n.x) > 0.9f ? mk(0.f, 1.f, 0.f) : mk(1.f, 0.f, 0.f));
+        o.b = b * __frsqrt_rn(dot(b, b));
+        o.t = cross(o.b, o.n);
+        const f3 d = mk(a.x, a.y, a.z) - v.p;
+        const f3 wo = to_local(o, d * __frsqrt_rn(dot(d, d)));
+        tl.put(w, kFon, o.n);
+        tl.put(w, kFob, o.b);
+        tl.put(w, kFwo, wo);
+        const float* c = m.kind == AR_MATERIAL_LAMBERTIAN ? m.albedo : m.f0;
+        tl.put(w, kFcol, m.kind == AR_MATERIAL_DIELECTRIC ? mk(m.eta, 0.f, 0.f) : mk(c[0], c[1], c[2]));
+        tl.at(w, kFalpha) = m.alpha;
+        tl.at(w, kFsmith) = smith_root(m.alpha, wo.z);
+        info |= m.kind << 28;
+    }
+    tl.at(w, kFinfo) = __uint_as_float(info);
+}
 
 // connect_bdpt for s >= 2 (:782-1044) + the t == 0 extension.  Emits a shadow
 // ray with the MIS-weighted contribution, or deposits directly when t == 0.
-// Camera-side data of strategy (s, *): z = z[s-1] and its shading frame.
-struct CamSide {
-    Vtx z;
-    f3 zp_p;
-    Onb oz;
-    MatView mz;
-    f3 wo_zl;
-};
-
-__device__ __forceinline__ CamSide cam_side(const BdParams& P, const BdJob& J, uint32_t si, uint32_t s) {
-    CamSide c;
-    c.z = load_vtx(P, 0, s - 1, si);
-    c.zp_p = load_vtx(P, 0, s - 2, si).p;
-    c.oz = onb_from_normal(c.z.n);
-    c.mz = vtx_mat(P, J, c.z, 0, s - 1, si);
-    c.wo_zl = to_local(c.oz, normalize(c.zp_p - c.z.p));
-    return c;
-}
-
-__device__ void connect_general(const BdParams& P, const BdJob& J, uint32_t job, uint32_t si, uint32_t S, uint32_t T,
-                                const MisCache& mc, bool lpt, const CamSide& cs, uint32_t s, uint32_t t,
-                                uint32_t pix) {
-    const Vtx& z = cs.z;
+// One direction serves both ends of a connection: the value, the density and
+// the geometry term of a strategy all take it and the two cosines.
+__device__ __forceinline__ void connect_general(const BdParams& P, const BdJob& J, const Tile& tl, uint32_t s,
+                                                uint32_t t) {
+    const uint32_t vz = tl.vertex(0, s - 1);
+    const f3 zp = tl.vec(vz, kFp), zn = tl.vec(vz, kFn);
     if (t == 0) {
-        const MatView& mz = cs.mz;
-        if (mz.emitter < 0 || !light_enabled(J.sc)) return;
-        const LightView lt = load_light(J.sc, uint32_t(mz.emitter));
-        const f3 wo = normalize(cs.zp_p - z.p);
+        const int32_t emitter = J.sc.materials[__float_as_uint(tl.at(vz, kFinfo)) & 0x0fffffffu].emitter;
+        if (emitter < 0 || !light_enabled(J.sc)) return;
+        const LightView lt = load_light(J.sc, uint32_t(emitter));
+        const f3 wo = normalize(tl.vec(vz - 1, kFp) - zp);
         if (dot(lt.n, wo) <= 0.f) return;
-        const f3 c = z.thr * lt.inten;
+        const f3 c = tl.vec(vz, kFthr) * lt.inten;
         if (max3(c) <= 0.f) return;
-        const float pdf_cc = light_pmf_of(J.sc, uint32_t(mz.emitter)) / lt.area;
-        const float w = mis_weight_cached(P, J, mc, si, S, T, s, 0, pdf_cc, 0.f, lpt);
-        film_add(J, pix, (c * w) * J.inv_spp);
+        const float pdf_cc = light_pmf_of(J.sc, uint32_t(emitter)) / lt.area;
+        film_add(J, tl.word(kIpix), (c * tile_mis(P, J, tl, s, 0, pdf_cc, 0.f)) * J.inv_spp);
         return;
     }
-    const Vtx y = load_vtx(P, 1, t - 1, si);
-    if (y.type == kTypeSurface && y.delta) return;
-    const f3 d = y.p - z.p;
+    const uint32_t vy = tl.vertex(1, t - 1);
+    const f3 yp = tl.vec(vy, kFp), yn = tl.vec(vy, kFn);
+    const f3 d = yp - zp;
     const float d2 = dot(d, d);
     if (d2 < 1e-10f) return;
-    const float dist = sqrtf(d2);
-    const f3 wi_z = d / dist;
-    const f3 wi_y = -wi_z;
-    const f3 so = z.p + (z.n * 1e-4f) * signum(dot(wi_z, z.n));
-    const f3 st = y.p + (y.n * 1e-4f) * signum(dot(wi_y, y.n));
-    const f3 sd = st - so;
-    const float sdist = length(sd);
-    if (sdist < 1e-6f) return;
-    const Onb& oz = cs.oz;
-    const MatView& mz = cs.mz;
-    const f3& wo_zl = cs.wo_zl;
-    const f3 f_z = bsdf_eval_ool(mz, to_local(oz, wi_z), wo_zl);
+    const float inv_dist = __frsqrt_rn(d2), inv_d2 = inv_dist * inv_dist;
+    const f3 wi_z = d * inv_dist;
+    const float dz = dot(wi_z, zn), dy = dot(-wi_z, yn);
+    const float4 ez = tile_bsdf(tl, vz, wi_z);
+    const f3 f_z = mk(ez.x, ez.y, ez.z);
     if (is_zero(f_z)) return;
-    f3 f_y = mk(1.f, 1.f, 1.f);
-    Onb oy;
-    MatView my;
-    f3 wo_yl = mk(0.f, 0.f, 0.f);
-    if (t != 1) {
-        oy = onb_from_normal(y.n);
-        my = vtx_mat(P, J, y, 1, t - 1, si);
-        const Vtx yp = load_vtx(P, 1, t - 2, si);
-        wo_yl = to_local(oy, normalize(yp.p - y.p));
-        f_y = bsdf_eval_ool(my, to_local(oy, wi_y), wo_yl);
-    }
-    if (is_zero(f_y)) return;
-    const float g = geometry_term(z.p, z.n, y.p, y.n);
+    const float cz = fabsf(dz), cy = fabsf(dy);
+    const f3 thr_z = tl.vec(vz, kFthr);
     f3 c;
+    float pdf_y;
     if (t == 1) {
-        const LightView L = load_light(J.sc, y.index);
+        const LightView L = load_light(J.sc, __float_as_uint(tl.at(vy, kFinfo)) & 0x0fffffffu);
         if (L.kind == AR_LIGHT_POINT) {
             // :951-967 — re-sample the point light toward z
             f3 lwi, lrad;
             float ldist, lpdf;
-            if (!light_sample(L, z.p, 0.f, 0.f, lwi, ldist, lrad, lpdf)) return;
-            const f3 f_direct = bsdf_eval_ool(mz, to_local(oz, lwi), wo_zl);
-            c = ((z.thr * f_direct) * fabsf(dot(z.n, lwi))) * lrad;
+            if (!light_sample(L, zp, 0.f, 0.f, lwi, ldist, lrad, lpdf)) return;
+            const float4 ed = tile_bsdf(tl, vz, lwi);
+            c = ((thr_z * mk(ed.x, ed.y, ed.z)) * fabsf(dot(zn, lwi))) * lrad;
         } else {
-            if (dot(y.n, wi_y) <= 0.f) return;
-            c = ((z.thr * f_z) * g) * y.thr;
+            if (dy <= 0.f) return;
+            c = ((thr_z * f_z) * (cz * cy * inv_d2)) * tl.vec(vy, kFthr);
         }
+        pdf_y = light_pdf_emission_dir(L, -wi_z);
     } else {
-        c = (((z.thr * f_z) * g) * f_y) * y.thr;
+        const float4 ey = tile_bsdf(tl, vy, -wi_z);
+        const f3 f_y = mk(ey.x, ey.y, ey.z);
+        if (is_zero(f_y)) return;
+        c = (((thr_z * f_z) * (cz * cy * inv_d2)) * f_y) * tl.vec(vy, kFthr);
+        pdf_y = ey.w;
     }
     if (max3(c) <= 0.f) return;
-    float pdf_cc;
-    if (t == 1) {
-        const LightView L = load_light(J.sc, y.index);
-        pdf_cc = pdf_sa_to_area(light_pdf_emission_dir(L, normalize(z.p - y.p)), y.p, z.p, z.n);
-    } else {
-        const f3 wiy = normalize(z.p - y.p);
-        pdf_cc = pdf_sa_to_area(bsdf_pdf_ool(my, to_local(oy, wiy), wo_yl), y.p, z.p, z.n);
-    }
-    const float pdf_cl = pdf_sa_to_area(bsdf_pdf_ool(mz, to_local(oz, normalize(y.p - z.p)), wo_zl), z.p, y.p, y.n);
-    const float w = mis_weight_cached(P, J, mc, si, S, T, s, t, pdf_cc, pdf_cl, lpt);
-    push_shadow(P, job, so, normalize(sd / sdist), sdist * (1.0f - 1e-4f), c * w, pix);
+    // the shadow ray, with the reference's operations
+    const f3 so = zp + (zn * 1e-4f) * signum(dz);
+    const f3 sd = (yp + (yn * 1e-4f) * signum(dy)) - so;
+    const float sdist = length(sd);
+    if (sdist < 1e-6f) return;
+    const float w = tile_mis(P, J, tl, s, t, pdf_y * cz * inv_d2, ez.w * cy * inv_d2);
+    push_shadow(P, tl.word(kIjob), so, normalize(sd / sdist), sdist * (1.0f - 1e-4f), c * w, tl.word(kIpix));
 }
 
 // connect_bdpt_s1 (:1051-1155): light tracing to the pinhole, splatted.
-__device__ void connect_s1(const BdParams& P, const BdJob& J, uint32_t job, uint32_t si, uint32_t S, uint32_t T, const MisCache& mc, bool lpt,
-                           uint32_t t) {
-    const Vtx y = load_vtx(P, 1, t - 1, si);
-    if (y.type == kTypeSurface && y.delta) return;
+__device__ __forceinline__ void connect_s1(const BdParams& P, const BdJob& J, const Tile& tl, uint32_t t) {
+    const uint32_t vy = tl.vertex(1, t - 1);
+    const f3 yp = tl.vec(vy, kFp), yn = tl.vec(vy, kFn);
     // PinholeCamera::sample_we (src/cameras.rs:175-240)
     const f3 co = ld3(J.cam.o);
-    const f3 to_cam0 = co - y.p;
+    const f3 to_cam0 = co - yp;
     const float d2 = dot(to_cam0, to_cam0);
     const float dist = sqrtf(d2);
     if (dist < 1e-6f) return;
@@ -610,21 +685,18 @@ __device__ void connect_s1(const BdParams& P, const BdJob& J, uint32_t job, uint
     if (px < 0.f || px >= float(J.width) || py < 0.f || py >= float(J.height)) return;
     const float c2 = ct * ct, c4 = c2 * c2;
     const float we = 1.0f / (J.cam.area * c4);
-    const Onb oy = onb_from_normal(y.n);
-    const MatView my = vtx_mat(P, J, y, 1, t - 1, si);
-    const Vtx yp = load_vtx(P, 1, t - 2, si);
-    const f3 wo_yl = to_local(oy, normalize(yp.p - y.p));
-    const f3 f_y = bsdf_eval_ool(my, to_local(oy, wi), wo_yl);
+    const float4 ey = tile_bsdf(tl, vy, wi);
+    const f3 f_y = mk(ey.x, ey.y, ey.z);
     if (is_zero(f_y)) return;
-    const float gf = fabsf(dot(y.n, wi)) / (dist * dist);
-    const f3 c = ((y.thr * f_y) * gf) * we;
+    const float dy = dot(yn, wi);
+    const float gf = fabsf(dy) / (dist * dist);
+    const f3 c = ((tl.vec(vy, kFthr) * f_y) * gf) * we;
     if (max3(c) <= 0.f) return;
-    const Vtx z0 = load_vtx(P, 0, 0, si);
-    const float pdf_cl = pdf_sa_to_area(bsdf_pdf_ool(my, to_local(oy, wi), wo_yl), y.p, co, z0.n);
-    const float w = mis_weight_cached(P, J, mc, si, S, T, 1, t, 0.f, pdf_cl, lpt);
+    const float pdf_cl = pdf_sa_to_area(ey.w, yp, co, tl.vec(tl.vertex(0, 0), kFn));
+    const float w = tile_mis(P, J, tl, 1, t, 0.f, pdf_cl);
     const uint32_t ix = min(uint32_t(px), J.width - 1), iy = min(uint32_t(py), J.height - 1);
-    const f3 o = y.p + (y.n * 1e-4f) * signum(dot(wi, y.n));
-    push_shadow(P, job, o, normalize(wi), dist * (1.0f - 1e-4f), c * w, iy * J.width + ix);
+    const f3 o = yp + (yn * 1e-4f) * signum(dy);
+    push_shadow(P, tl.word(kIjob), o, normalize(wi), dist * (1.0f - 1e-4f), c * w, iy * J.width + ix);
 }
 
 // Counting sort of the batch samples by their subpath lengths (S, T), so the
@@ -684,54 +756,85 @@ __global__ void __launch_bounds__(256) k_bd_scatter(BdParams P) {
     }
 }
 
-// Copies every sample's vertices to its sorted position oi (reads scattered,
-// writes coalesced), so k_bd_connect, whose thread oi handles sample
-// order[oi], reads vertex k of 32 consecutive samples as one contiguous block.
-// One thread per (depth k, position oi), oi fastest: a warp copies depth k of
-// 32 consecutive positions, and many independent copies are in flight.
-__global__ void __launch_bounds__(256) k_bd_permute(BdParams P) {
+__global__ void __launch_bounds__(kConnectThreads, kConnectBlocks) k_bd_connect(BdParams P, uint32_t maxv, uint32_t samples) {
+    extern __shared__ double tile_mem[];
+    Tile tl;
+    tl.maxv = maxv;
+    tl.samples = samples;
+    tl.pre = tile_mem;
+    tl.inv = tl.pre + 2 * maxv * samples;
+    tl.f = reinterpret_cast<float*>(tl.inv + 2 * maxv * samples);
+    tl.i = reinterpret_cast<uint32_t*>(tl.f + 2 * maxv * kTileFields * samples);
+    tl.lane = threadIdx.x & (samples - 1u);
+    const uint32_t row = threadIdx.x / samples, rows = kConnectThreads / samples;
     const uint32_t ns = P.dyn[0];
-    const uint64_t total = uint64_t(ns) * P.maxv;
-    for (uint64_t w = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; w < total;
-         w += uint64_t(gridDim.x) * blockDim.x) {
-        const uint32_t k = uint32_t(w / ns), oi = uint32_t(w - uint64_t(k) * ns);
-        const uint32_t si = P.order[oi];
-        for (uint32_t sub = 0; sub < 2; ++sub) {
-            if (k >= P.nv[sub * P.cap + si]) continue;
-            const size_t from = vidx(P, sub, k, si), to = vidx(P, sub, k, oi);
-            P.sva[to] = P.va[from];
-            P.svb[to] = P.vb[from];
-            const float4 c = P.vc[from];
-            P.svc[to] = c;
-            if ((__float_as_uint(c.w) >> 28) & 1u) P.svuv[to] = P.vuv[from];  // textured vertices only
+    for (uint32_t tile = blockIdx.x * samples; tile < ns; tile += gridDim.x * samples) {
+        if (threadIdx.x < samples) {
+            const uint32_t oi = tile + threadIdx.x;
+            uint32_t S = 0, T = 0, job = 0, pix = 0, si = 0, flags = 0;
+            if (oi < ns) {
+                si = P.order[oi];
+                job = P.sjob[si];
+                const BdJob& J = P.jobs[job];
+                S = P.nv[si];
+                T = P.nv[P.cap + si];
+                pix = uint32_t(P.sindex[si] % (J.width * J.height));
+                if (J.mis_mode == AR_MIS_POWER && J.mis_beta == 2.0f && S <= kMisCache && T <= kMisCache)
+                    flags |= kFlagFastMis;
+                if (T >= 1 && J.sc.lights[load_vtx(P, 1, 0, si).index].kind == AR_LIGHT_POINT) flags |= kFlagPointLight;
+            }
+            tl.word(kIs) = S;
+            tl.word(kIt) = T;
+            tl.word(kIjob) = job;
+            tl.word(kIpix) = pix;
+            tl.word(kIsample) = si;
+            tl.word(kIflags) = flags;
         }
-    }
-}
-
-// One thread per sample: the MIS prefix sums are built once, then the
-// strategies run camera-vertex-major so each z's frame is computed once.
-__global__ void __launch_bounds__(128) k_bd_connect(BdParams P) {
-    // P.va/vb/vc are the sorted copies here (see bdpt_run_batch): vertex
-    // records of sample order[oi] are read at index oi; the per-sample arrays
-    // (job, lengths, global index) stay indexed by the sample itself.
-    const uint32_t ns = P.dyn[0];
-    for (uint32_t oi = blockIdx.x * blockDim.x + threadIdx.x; oi < ns; oi += gridDim.x * blockDim.x) {
-        const uint32_t si = P.order[oi];
-        const uint32_t job = P.sjob[si];
-        const BdJob& J = P.jobs[job];
-        const uint32_t S = P.nv[si], T = P.nv[P.cap + si];
-        const uint32_t pix = uint32_t(P.sindex[si] % (J.width * J.height));
+        __syncthreads();
+        const uint32_t S = tl.word(kIs), T = tl.word(kIt), si = tl.word(kIsample);
+        const BdJob& J = P.jobs[tl.word(kIjob)];
+        for (uint32_t v = row; v < 2 * maxv; v += rows) {
+            const uint32_t sub = v >= maxv ? 1u : 0u, k = v - sub * maxv;
+            if (k < (sub ? T : S)) tile_load(P, J, tl, sub, k, si);
+        }
+        __syncthreads();
+        if (row < 2) {  // C_s and D_t from the q^2 (rows 0 and 1: camera and light side)
+            const uint32_t n = row ? T : S;
+            double c = 1.0;
+            for (uint32_t k = 0; k < n; ++k) {
+                double& x = tl.prefix(tl.vertex(row, k));
+                if (k >= 1) c = 1.0 + x * c;
+                x = c;
+            }
+        }
+        // the tile's longest subpaths bound the strategy loop of all its rows
+        uint32_t sm = S, tm = T;
+        for (uint32_t o = 16; o > 0; o >>= 1) {
+            sm = max(sm, __shfl_xor_sync(0xffffffffu, sm, o));
+            tm = max(tm, __shfl_xor_sync(0xffffffffu, tm, o));
+        }
+        __syncthreads();
+        // strategies, like ones together: s >= 2 with t >= 2, t = 1, t = 0, then s = 1
         const uint32_t limit = J.max_depth + 2;
-        MisCache mc;
-        build_mis_cache(P, J, oi, S, T, mc);
-        bool lpt = false;
-        if (T >= 1) lpt = J.sc.lights[load_vtx(P, 1, 0, oi).index].kind == AR_LIGHT_POINT;
-        if (S >= 1)
-            for (uint32_t t = 2; t <= T && 1 + t <= limit; ++t) connect_s1(P, J, job, oi, S, T, mc, lpt, t);
-        for (uint32_t s = 2; s <= S; ++s) {
-            const CamSide cs = cam_side(P, J, oi, s);
-            for (uint32_t t = 0; t <= T && s + t <= limit; ++t) connect_general(P, J, job, oi, S, T, mc, lpt, cs, s, t, pix);
+        const uint32_t ns2 = sm >= 2 ? sm - 1 : 0, nt2 = tm >= 2 ? tm - 1 : 0, both = ns2 * nt2;
+        const uint32_t total = both + 2 * ns2 + (sm >= 1 ? nt2 : 0);
+        for (uint32_t e = row; e < total; e += rows) {
+            uint32_t s, t;
+            if (e < both) {
+                s = 2 + e / nt2;
+                t = 2 + e % nt2;
+            } else if (e < both + 2 * ns2) {
+                t = e < both + ns2 ? 1 : 0;
+                s = 2 + (e - both) - (t ? 0 : ns2);
+            } else {
+                s = 1;
+                t = 2 + (e - both - 2 * ns2);
+            }
+            if (s > S || t > T || s + t > limit) continue;
+            if (s == 1) connect_s1(P, J, tl, t);
+            else connect_general(P, J, tl, s, t);
         }
+        __syncthreads();
     }
 }
 
@@ -803,7 +906,7 @@ struct BdptBatcher {
 
 size_t bdpt_batch_bytes(uint32_t max_depth, uint32_t batch) {
     const size_t maxv = max_depth + 1;
-    const size_t per_sample = 2 * 2 * maxv * 56 + 2 + 2 * (16 + 4) + 2 * 2 * (32 + 4) + 2 * 20 + 4 + 8 +
+    const size_t per_sample = 2 * maxv * 56 + 2 + 2 * (16 + 4) + 2 * 2 * (32 + 4) + 2 * 20 + 4 + 8 +
                               size_t(max_pairs_for(max_depth)) * 52 + 4;
     return per_sample * batch + 64 * 1024;
 }
@@ -812,6 +915,7 @@ BdptBatcher* bdpt_create(ar_context* ctx, uint32_t max_depth_cap, uint32_t batch
     AR_REQUIRE(max_depth_cap <= 62, AR_ERR_INVALID_ARGUMENT, "BDPT max_depth must be <= 62");
     auto b = std::make_unique<BdptBatcher>();
     b->ctx = ctx;
+    AR_CUDA(cudaFuncSetAttribute(k_bd_connect, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTileMax)));
     b->max_depth_cap = max_depth_cap;
     b->batch = batch;
     b->mem.alloc(bdpt_batch_bytes(max_depth_cap, batch));
@@ -831,10 +935,6 @@ BdptBatcher* bdpt_create(ar_context* ctx, uint32_t max_depth_cap, uint32_t batch
     P.vb = carve<float4>(cur, nvtx);
     P.vc = carve<float4>(cur, nvtx);
     P.vuv = carve<float2>(cur, nvtx);
-    P.sva = carve<float4>(cur, nvtx);
-    P.svb = carve<float4>(cur, nvtx);
-    P.svc = carve<float4>(cur, nvtx);
-    P.svuv = carve<float2>(cur, nvtx);
     P.nv = carve<uint8_t>(cur, 2 * size_t(batch));
     P.thr = carve<float4>(cur, 2 * size_t(batch));
     P.dim = carve<uint32_t>(cur, 2 * size_t(batch));
@@ -907,18 +1007,10 @@ static uint32_t launch_batch(BdptBatcher* b, uint32_t max_depth, cudaStream_t s)
         k_bd_scatter<<<g, 256, 0, s>>>(P);
     }
     {
-        KernelScope ks(ctx->prof, s, "bdpt_permute");
-        k_bd_permute<<<g, 256, 0, s>>>(P);
-    }
-    {
         KernelScope ks(ctx->prof, s, "bdpt_connect");
-        BdParams Pc = P;
-        Pc.va = P.sva;
-        Pc.vb = P.svb;
-        Pc.vc = P.svc;
-        Pc.vuv = P.svuv;
-        k_bd_connect<<<std::max(1, int(std::min<uint64_t>((b->batch + 127) / 128, ctx->num_sms * 16))), 128, 0,
-                       s>>>(Pc);
+        const uint32_t maxv = max_depth + 1, samples = tile_samples(maxv);
+        k_bd_connect<<<std::max(1, int(std::min<uint64_t>((b->batch + samples - 1) / samples, ctx->num_sms * kConnectBlocks))),
+                       kConnectThreads, tile_bytes(maxv, samples), s>>>(P, maxv, samples);
     }
     {
         KernelScope ks(ctx->prof, s, "bdpt_shadow");
@@ -926,9 +1018,9 @@ static uint32_t launch_batch(BdptBatcher* b, uint32_t max_depth, cudaStream_t s)
     }
     k_bd_count<<<1, 32, 0, s>>>(P.counts, max_depth, ctx->stats_d.as<unsigned long long>(), err);
     AR_CUDA(cudaGetLastError());
-    // generate, (extend, vertex) per depth, hist/scan/scatter, permute,
-    // connect, shadow, count
-    return 2 * max_depth + 8;
+    // generate, (extend, vertex) per depth, hist/scan/scatter, connect,
+    // shadow, count
+    return 2 * max_depth + 7;
 }
 
 uint32_t bdpt_run_batch(BdptBatcher* b, const std::vector<BdJob>& jobs, const std::vector<BdSegment>& segs,
@@ -978,7 +1070,7 @@ uint32_t bdpt_run_batch(BdptBatcher* b, const std::vector<BdJob>& jobs, const st
         AR_CUDA(e);
     }
     AR_CUDA(cudaGraphLaunch(ge, st));
-    return 2 * max_depth + 8;
+    return 2 * max_depth + 7;
 }
 
 BdJob make_bdpt_job(const ar_scene* sc, const CameraDev& cam, const ar_integrator_cfg& cfg, uint32_t w, uint32_t h,
@@ -1009,7 +1101,9 @@ void render_bdpt_film(ar_context* ctx, const ar_scene* sc, const CameraDev& cam,
     const uint64_t first = npix * s0, total = npix * (s1 - s0);
     const size_t budget = ctx->bdpt_budget;
     const size_t per = bdpt_batch_bytes(cfg.max_depth, 1024) / 1024 + 1;
-    const uint32_t batch = uint32_t(std::max<uint64_t>(1024, std::min<uint64_t>(total, budget / per)));
+    const uint64_t fit = std::max<uint64_t>(1024, budget / per);
+    const uint64_t count = (total + fit - 1) / fit;  // batches, of equal size
+    const uint32_t batch = uint32_t(std::max<uint64_t>(1024, (total + count - 1) / count));
     const auto fits = [&](const BdptBatcher* b) {
         return b && bdpt_max_depth_cap(b) >= cfg.max_depth && bdpt_batch_capacity(b) >= batch;
     };
@@ -1019,7 +1113,7 @@ void render_bdpt_film(ar_context* ctx, const ar_scene* sc, const CameraDev& cam,
         ctx->bdpt = nullptr;
         ctx->bdpt = bdpt_create(ctx, std::max(cfg.max_depth, 10u), batch);
     }
-    const uint32_t cap = bdpt_batch_capacity(ctx->bdpt);
+    const uint32_t cap = batch;
     // Renders of two or more batches alternate them over two lanes (the
     // context stream and a second stream, each with its own batch buffers):
     // one batch's stage tails overlap the other's work.  Profiling keeps one
@@ -1030,7 +1124,7 @@ void render_bdpt_film(ar_context* ctx, const ar_scene* sc, const CameraDev& cam,
             AR_CUDA(cudaStreamCreateWithFlags(&ctx->lane_stream, cudaStreamNonBlocking));
             for (cudaEvent_t& e : ctx->lane_ev) AR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         }
-        if (!fits(ctx->bdpt2) || bdpt_batch_capacity(ctx->bdpt2) < cap) {
+        if (!fits(ctx->bdpt2)) {
             AR_CUDA(cudaStreamSynchronize(ctx->lane_stream));
             bdpt_destroy(ctx->bdpt2);
             ctx->bdpt2 = nullptr;

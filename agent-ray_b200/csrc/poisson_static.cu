@@ -26,9 +26,9 @@
 
 namespace ar {
 
-void poisson_sor_with_scratch(cudaStream_t stream, int num_sms, const ar_integrator_cfg& cfg, uint32_t w, uint32_t h,
-                              const float* primal, const float* gx, const float* gy, float* rhs, float* img,
-                              float* out);
+uint64_t poisson_sor_with_scratch(cudaStream_t stream, int num_sms, const ar_integrator_cfg& cfg, uint32_t w,
+                                  uint32_t h, const float* primal, const float* gx, const float* gy, float* rhs,
+                                  float* img, float* out);
 
 namespace {
 

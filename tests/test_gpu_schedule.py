@@ -86,3 +86,19 @@ def test_bdpt_connection_tiles_match_oracle(ctx, depth, mode, beta):
     gpu = out.reshape(h, w, 3).astype(np.float64)
     assert np.isfinite(gpu).all() and gpu.max() > 0
     np.testing.assert_allclose(gpu, ref, rtol=1e-3, atol=1e-3 * ref.mean())
+
+
+@pytest.mark.parametrize("h,w,iters", [(1, 1, 200), (1, 70, 7), (65, 1, 5), (16, 16, 12), (193, 193, 13), (300, 500, 1),
+                                       (517, 519, 11), (700, 640, 0)])
+def test_sor_regions_are_bit_exact(ctx, h, w, iters):
+    # Images of one region and of many, ragged against every overlap the solver
+    # chooses (24 rings for small images down to 10), odd launch counts and a
+    # last launch of fewer sweeps, against the oracle's sequential red-black SOR.
+    import oracle as O
+    rng = np.random.default_rng(h * 1000 + w)
+    primal = rng.uniform(0.0, 2.0, (h, w, 3)).astype(np.float32)
+    gx = (rng.normal(size=(h, w, 3)) * 0.2).astype(np.float32)
+    gy = (rng.normal(size=(h, w, 3)) * 0.2).astype(np.float32)
+    ref = O.poisson_sor_f32(primal, gx, gy, 0.2, iters, 1.6)
+    out, _ = agentray.poisson_reconstruct(ctx, primal, gx, gy, 0.2, A.POISSON_SOR, iters, 1.6)
+    np.testing.assert_array_equal(out, ref)

@@ -171,6 +171,9 @@ __global__ void k_clamp(size_t n, const float* __restrict__ in, float* __restric
 }
 
 // ---- CG ----
+// A sum over the image is spread over this many places (3 channels each).
+constexpr uint32_t kCgSlots = 16, kCgSum = 3 * kCgSlots;
+
 template <class T>
 __device__ __forceinline__ void stencil(uint32_t w, uint32_t h, uint32_t i, const T* v, double alpha, double out[3]) {
     const uint32_t x = i % w, y = i / w;
@@ -204,7 +207,12 @@ __device__ __forceinline__ void block_add3(double a0, double a1, double a2, doub
             a1 += __shfl_down_sync(0xffffffffu, a1, o);
             a2 += __shfl_down_sync(0xffffffffu, a2, o);
         }
-        if (lane == 0) { atomicAdd(dst, a0); atomicAdd(dst + 1, a1); atomicAdd(dst + 2, a2); }
+        if (lane == 0) {
+            dst += 3 * (blockIdx.x % kCgSlots);
+            atomicAdd(dst, a0);
+            atomicAdd(dst + 1, a1);
+            atomicAdd(dst + 2, a2);
+        }
     }
     __syncthreads();
 }
@@ -231,9 +239,9 @@ __global__ void k_cg_setup(uint32_t w, uint32_t h, const float* primal, const fl
     block_add3(a[0], a[1], a[2], bb);
 }
 
-// r (f32) = b - A x (f64 arithmetic); p = r; d = 0; rr += |r|^2 (f64).
+// r (f32) = b - A x (f64 arithmetic); d = 0; rr += |r|^2 (f64).
 __global__ void k_cg_residual(uint32_t w, uint32_t h, const double* b, const double* x, double alpha, float* r,
-                              float* p, float* d, double* rr) {
+                              float* d, double* rr) {
     const uint32_t n = w * h;
     double a[3] = {0, 0, 0};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -242,7 +250,6 @@ __global__ void k_cg_residual(uint32_t w, uint32_t h, const double* b, const dou
         for (int c = 0; c < 3; ++c) {
             const double rv = b[3 * i + c] - ax[c];
             r[3 * i + c] = float(rv);
-            p[3 * i + c] = float(rv);
             d[3 * i + c] = 0.f;
             a[c] += rv * rv;
         }
@@ -250,52 +257,134 @@ __global__ void k_cg_residual(uint32_t w, uint32_t h, const double* b, const dou
     block_add3(a[0], a[1], a[2], rr);
 }
 
-// q = A p (f32 storage, f64 accumulation); pq += p.q
-__global__ void k_cg_matvec(uint32_t w, uint32_t h, const float* p, double alpha, float* q, double* pq) {
-    const uint32_t n = w * h;
-    double a[3] = {0, 0, 0};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double ap[3];
-        stencil(w, h, i, p, alpha, ap);
-        for (int c = 0; c < 3; ++c) {
-            q[3 * i + c] = float(ap[c]);
-            a[c] += double(p[3 * i + c]) * ap[c];
-        }
-    }
-    block_add3(a[0], a[1], a[2], pq);
+// ---- the CG iteration ----
+// Two kernels an iteration.  The arrays of an image do not fit the L1s, and half
+// of an SM's L2 accesses go to the other die, so an iteration is bound by its
+// passes over L2: 13 of them when direction, product and update were kernels of
+// their own, 8 here (the first forms p = r + beta p for a float and its
+// neighbours, stores p and sums p.Ap; the second forms A p again from p instead of
+// storing it).  A thread owns one float column (a pixel column's channel) and
+// walks down `rows` rows, so the vertical neighbours stay in registers, already
+// widened; the horizontal ones come through L1.  The sums of a block go to one of
+// kCgSlots places, so that hundreds of blocks do not queue on three addresses.
+// Every float goes through the same operations as before: f64 stencil and
+// sums, f32 vectors.  A solve to 1e-6 (64 iterations): 1024x1024 3.00 -> 2.08
+// ms, 512x512 1.87 -> 1.13, 256x256 1.19 -> 0.92.  Not faster: tiles with a rim in shared memory (2.7
+// ms at 1024x1024: their index arithmetic), loads batched four rows ahead (2.4),
+// four floats a thread with neighbours by shuffle (2.6).
+constexpr uint32_t kCgThreads = 192, kCgInner = 32;  // 64 pixels of a row
+
+// Rows a thread walks: fewer halo rows and prologues the more there are, as
+// long as five blocks an SM are left (16 rows against 8, 4 at 1024x1024: 2.12,
+// 2.34, 2.51 ms; 4 against 8, 16 at 512x512: 1.16, 1.27, 1.73; 2 against 4, 8 at
+// 256x256: 0.87, 0.93, 1.15).
+uint32_t cg_rows(uint32_t w, uint32_t h, int num_sms) {
+    const uint64_t cols = (3 * uint64_t(w) + kCgThreads - 1) / kCgThreads;
+    uint32_t rows = 16;
+    while (rows > 1 && cols * ((h + rows - 1) / rows) < uint64_t(5 * num_sms)) rows /= 2;
+    while ((h + rows - 1) / rows > 65535u) rows *= 2;  // the grid's y extent
+    return rows;
 }
 
-// scal layout (f64): [0..3) rr, [3..6) pq, [6..9) rr_new
-__global__ void k_cg_update(uint32_t n, const float* p, const float* q, float* d, float* r, const double* scal,
-                            double* rr_new) {
-    float al[3];
-    for (int c = 0; c < 3; ++c) al[c] = scal[3 + c] != 0.0 ? float(scal[c] / scal[3 + c]) : 0.f;
-    double a[3] = {0, 0, 0};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        for (int c = 0; c < 3; ++c) {
-            d[3 * i + c] += al[c] * p[3 * i + c];
-            const float rv = r[3 * i + c] - al[c] * q[3 * i + c];
-            r[3 * i + c] = rv;
-            a[c] += double(rv) * double(rv);
-        }
+// coef[c] = num / den of channel c (0 where den is 0), from the slots of the two
+// sums: warp c adds up channel c.  Visible to the block after its next barrier.
+// (Plain loads: the sums are complete, and one copy in L1 serves all the blocks
+// of an SM; read past L1 by every thread, these few lines cost 300 us.)
+__device__ __forceinline__ void cg_ratio(const double* num, const double* den, float coef[3]) {
+    const uint32_t warp = threadIdx.x / 32u, lane = threadIdx.x & 31u;
+    if (warp >= 3) return;
+    double a = lane < kCgSlots ? num[3 * lane + warp] : 0.0, b = lane < kCgSlots ? den[3 * lane + warp] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
     }
-    block_add3(a[0], a[1], a[2], rr_new);
+    if (lane == 0) coef[warp] = b != 0.0 ? float(a / b) : 0.f;
 }
 
-__global__ void k_cg_direction(uint32_t n, const float* r, float* p, const double* scal) {
-    float be[3];
-    for (int c = 0; c < 3; ++c) be[c] = scal[c] != 0.0 ? float(scal[6 + c] / scal[c]) : 0.f;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        for (int c = 0; c < 3; ++c) p[3 * i + c] = r[3 * i + c] + be[c] * p[3 * i + c];
+// Adds each thread's `a`, of channel threadIdx.x % 3, to the block's slot of `sum`.
+__device__ __forceinline__ void cg_add(double a, double* sum) {
+    __shared__ double part[kCgThreads];
+    part[threadIdx.x] = a;
+    __syncthreads();
+    const uint32_t warp = threadIdx.x / 32u, lane = threadIdx.x & 31u;
+    if (warp < 3) {  // warp c adds up channel c
+        double t = part[3 * lane + warp] + part[96 + 3 * lane + warp];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) atomicAdd(sum + 3 * ((blockIdx.x + blockIdx.y * gridDim.x) % kCgSlots) + warp, t);
+    }
 }
 
-// rr <- rr_new; pq, rr_new <- 0
-__global__ void k_cg_rotate(double* scal) {
-    if (threadIdx.x < 3) {
-        scal[threadIdx.x] = scal[6 + threadIdx.x];
-        scal[3 + threadIdx.x] = 0.0;
-        scal[6 + threadIdx.x] = 0.0;
+// Calls each(i, v, A v) for the floats of this thread's column in its rows;
+// at(i) gives v of float i (f32).
+template <class At, class Each>
+__device__ __forceinline__ void cg_walk(uint32_t w, uint32_t h, uint32_t rows, double alpha, At at, Each each) {
+    const uint32_t f = blockIdx.x * kCgThreads + threadIdx.x, pitch = 3u * w;
+    const uint32_t y0 = blockIdx.y * rows, y1 = min(h, y0 + rows);
+    if (f >= pitch || y0 >= h) return;
+    const bool left = f >= 3u, right = f + 3u < pitch;
+    const int nx = int(left) + int(right);
+    uint32_t i = y0 * pitch + f;
+    float m32 = at(i);
+    double up = y0 > 0 ? double(at(i - pitch)) : 0.0, mid = double(m32);
+#pragma unroll 4
+    for (uint32_t y = y0; y < y1; ++y, i += pitch) {
+        const float d32 = y + 1 < h ? at(i + pitch) : 0.f;
+        const float l32 = left ? at(i - 3u) : 0.f, r32 = right ? at(i + 3u) : 0.f;
+        const double down = double(d32);
+        double s = double(l32);  // left, right, up, down; outside the image 0
+        s += double(r32);
+        s += up;
+        s += down;
+        const double diag = alpha + (nx + int(y > 0) + int(y + 1 < h));
+        each(i, m32, diag * mid - s);
+        up = mid;
+        mid = down;
+        m32 = d32;
     }
+}
+
+// p = r + beta p (beta = rr / rr_prev; the first iteration takes p = r), pq += p.Ap
+__global__ void __launch_bounds__(kCgThreads) k_cg_direction(uint32_t w, uint32_t h, uint32_t rows,
+                                                             const float* __restrict__ r,
+                                                             const float* __restrict__ p_in, float* __restrict__ p_out,
+                                                             double alpha, const double* __restrict__ rr,
+                                                             const double* __restrict__ rr_prev, double* pq) {
+    __shared__ float coef[3];
+    double a = 0.0;
+    const auto each = [&](uint32_t i, float p, double ap) {
+        p_out[i] = p;
+        a += double(p) * ap;
+    };
+    if (rr_prev) {
+        cg_ratio(rr, rr_prev, coef);
+        __syncthreads();
+        const float be = coef[threadIdx.x % 3u];
+        cg_walk(w, h, rows, alpha, [&](uint32_t i) { return r[i] + be * p_in[i]; }, each);
+    } else {
+        cg_walk(w, h, rows, alpha, [&](uint32_t i) { return r[i]; }, each);
+    }
+    cg_add(a, pq);
+}
+
+// d += al p, r -= al (A p), al = rr / pq; rr_new += r.r
+__global__ void __launch_bounds__(kCgThreads) k_cg_update(uint32_t w, uint32_t h, uint32_t rows,
+                                                          const float* __restrict__ p, float* __restrict__ d,
+                                                          float* __restrict__ r, double alpha,
+                                                          const double* __restrict__ rr,
+                                                          const double* __restrict__ pq, double* rr_new) {
+    __shared__ float coef[3];
+    cg_ratio(rr, pq, coef);
+    __syncthreads();
+    const float al = coef[threadIdx.x % 3u];
+    double a = 0.0;
+    cg_walk(w, h, rows, alpha, [&](uint32_t i) { return p[i]; },
+            [&](uint32_t i, float pv, double ap) {
+                d[i] += al * pv;
+                const float rv = r[i] - al * float(ap);
+                r[i] = rv;
+                a += double(rv) * double(rv);
+            });
+    cg_add(a, rr_new);
 }
 
 __global__ void k_cg_accumulate(size_t n, double* x, const float* d) {
@@ -364,45 +453,51 @@ uint64_t poisson_reconstruct(ar_context* ctx, const ar_integrator_cfg& cfg, uint
     const double alpha = double(cfg.alpha);
     const double tol = cfg.poisson_tolerance > 0 ? cfg.poisson_tolerance : 1e-6;
     const uint32_t max_total = cfg.poisson_iterations ? cfg.poisson_iterations : 1000;
-    const uint32_t inner = 32;
-    ctx->solver.ensure(3 * n * (2 * sizeof(double) + 4 * sizeof(float)) + 16 * sizeof(double) + 1024);
+    // sums: |b|^2, rr of iterations 0..kCgInner, pq of 0..kCgInner - 1
+    const size_t sums = (2 * kCgInner + 2) * kCgSum * sizeof(double);
+    ctx->solver.ensure(3 * n * (2 * sizeof(double) + 4 * sizeof(float)) + sums + 1024);
     double* b = ctx->solver.buf.as<double>();
     double* x = b + 3 * n;
     float* r = reinterpret_cast<float*>(x + 3 * n);
-    float* p = r + 3 * n;
-    float* q = p + 3 * n;
-    float* d = q + 3 * n;
-    double* scal = reinterpret_cast<double*>(d + 3 * n + 64);
-    scal = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(scal) + 63) & ~uintptr_t(63));
-    double* bb = scal + 9;
-    AR_CUDA(cudaMemsetAsync(scal, 0, 16 * sizeof(double), st));
+    float* p[2] = {r + 3 * n, r + 6 * n};
+    float* d = r + 9 * n;
+    double* bb = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(d + 3 * n) + 63) & ~uintptr_t(63));
+    double* rr = bb + kCgSum;
+    double* pq = rr + (kCgInner + 1) * kCgSum;
+    AR_CUDA(cudaMemsetAsync(bb, 0, kCgSum * sizeof(double), st));
     k_cg_setup<<<grid, 256, 0, st>>>(w, h, primal, gx, gy, alpha,
                                      (cfg.gdpt_flags & AR_GDPT_CONSISTENT_DIVERGENCE) != 0, b, x, bb);
-    double hb[16];
+    const uint32_t rows = cg_rows(w, h, ctx->num_sms);
+    const dim3 blocks((3 * w + kCgThreads - 1) / kCgThreads, (h + rows - 1) / rows);
+    double hb[2 * kCgSum];
     double res = 0.0;
     uint32_t total = 0;
     uint64_t launches = 1;
     for (;;) {
-        AR_CUDA(cudaMemsetAsync(scal, 0, 9 * sizeof(double), st));
-        k_cg_residual<<<grid, 256, 0, st>>>(w, h, b, x, alpha, r, p, d, scal);
+        AR_CUDA(cudaMemsetAsync(rr, 0, sums - kCgSum * sizeof(double), st));
+        k_cg_residual<<<grid, 256, 0, st>>>(w, h, b, x, alpha, r, d, rr);
         launches++;
-        AR_CUDA(cudaMemcpyAsync(hb, scal, 12 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        AR_CUDA(cudaMemcpyAsync(hb, bb, 2 * kCgSum * sizeof(double), cudaMemcpyDeviceToHost, st));
         AR_CUDA(cudaStreamSynchronize(st));
         res = 0.0;
-        for (int c = 0; c < 3; ++c) {
-            const double bn = hb[9 + c] > 0 ? std::sqrt(hb[9 + c]) : 1.0;
-            res = std::max(res, std::sqrt(hb[c]) / bn);
+        for (uint32_t c = 0; c < 3; ++c) {
+            double sb = 0.0, sr = 0.0;
+            for (uint32_t k = 0; k < kCgSlots; ++k) {
+                sb += hb[3 * k + c];
+                sr += hb[kCgSum + 3 * k + c];
+            }
+            res = std::max(res, std::sqrt(sr) / (sb > 0 ? std::sqrt(sb) : 1.0));
         }
         if (res <= tol || total >= max_total) break;
-        for (uint32_t k = 0; k < inner; ++k) {
-            k_cg_matvec<<<grid, 256, 0, st>>>(w, h, p, alpha, q, scal + 3);
-            k_cg_update<<<grid, 256, 0, st>>>(uint32_t(n), p, q, d, r, scal, scal + 6);
-            k_cg_direction<<<grid, 256, 0, st>>>(uint32_t(n), r, p, scal);
-            k_cg_rotate<<<1, 32, 0, st>>>(scal);
+        for (uint32_t k = 0; k < kCgInner; ++k) {
+            double *rr_k = rr + k * kCgSum, *pq_k = pq + k * kCgSum;
+            k_cg_direction<<<blocks, kCgThreads, 0, st>>>(w, h, rows, r, p[(k + 1) & 1], p[k & 1], alpha, rr_k,
+                                                          k ? rr_k - kCgSum : nullptr, pq_k);
+            k_cg_update<<<blocks, kCgThreads, 0, st>>>(w, h, rows, p[k & 1], d, r, alpha, rr_k, pq_k, rr_k + kCgSum);
         }
-        total += inner;
+        total += kCgInner;
         k_cg_accumulate<<<grid, 256, 0, st>>>(3 * n, x, d);
-        launches += 4 * inner + 1;
+        launches += 2 * kCgInner + 1;
     }
     k_cg_output<<<grid, 256, 0, st>>>(3 * n, x, out);
     AR_CUDA(cudaGetLastError());

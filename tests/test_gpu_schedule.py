@@ -102,3 +102,26 @@ def test_sor_regions_are_bit_exact(ctx, h, w, iters):
     ref = O.poisson_sor_f32(primal, gx, gy, 0.2, iters, 1.6)
     out, _ = agentray.poisson_reconstruct(ctx, primal, gx, gy, 0.2, A.POISSON_SOR, iters, 1.6)
     np.testing.assert_array_equal(out, ref)
+
+
+@pytest.mark.parametrize("h,w", [(1, 1), (1, 130), (70, 1), (33, 64), (64, 65), (259, 200)])
+def test_cg_sizes_reach_the_exact_solution(ctx, h, w):
+    # Images narrower than a block of columns, ragged last blocks and row runs of
+    # every length the solver chooses.  |x - x*| <= |b - A x| / lambda_min, with
+    # lambda_min = alpha = 0.2 and |b - A x| <= 1e-6 |b|; plus the f32 output.
+    import oracle as O
+    rng = np.random.default_rng(h * 1000 + w)
+    primal = rng.uniform(0.0, 2.0, (h, w, 3)).astype(np.float32)
+    gx = (rng.normal(size=(h, w, 3)) * 0.2).astype(np.float32)
+    gy = (rng.normal(size=(h, w, 3)) * 0.2).astype(np.float32)
+    gx[:, -1] = 0
+    gy[-1, :] = 0
+    exact, _ = O.poisson_exact_f64(primal, gx, gy, 0.2)
+    out, res = agentray.poisson_reconstruct(ctx, primal, gx, gy, 0.2, A.POISSON_CG, 2000, 1.6, 1e-6)
+    assert 0 <= res <= 1e-6
+    div = gx.astype(np.float64) + gy
+    div[:, 1:] -= gx[:, :-1]
+    div[1:] -= gy[:-1]
+    b = np.linalg.norm((0.2 * primal.astype(np.float64) + div).reshape(-1, 3), axis=0)
+    want = np.maximum(exact, 0)
+    assert np.all(np.abs(out - want) <= 5e-6 * b + 2e-7 * np.abs(want))

@@ -1,10 +1,11 @@
 // Film output on the device: Film::to_rgb_image (src/film.rs:276-302) with
-// tonemap_pixel (:153-181).  One thread per pixel; every multiply and add is
+// tonemap_pixel (:153-181); every multiply and add is
 // rounded separately in the reference's order (this file is compiled with
 // -fmad=false), the divisions are IEEE, and powf is CUDA's (within 2 ulp of
 // the host libm, so an 8-bit value can differ by one where the encoded value
 // sits on a rounding boundary).
 #include <algorithm>
+#include <cfloat>
 #include <cstdio>
 #include <cstring>
 #include <thread>
@@ -23,31 +24,100 @@ __device__ __forceinline__ float luminance(float r, float g, float b) {
     return (0.2126f * r + 0.7152f * g) + 0.0722f * b;
 }
 
+__device__ __forceinline__ float log2f_approx(float x) {
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float exp2f_approx(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 __device__ __forceinline__ uint8_t to_u8(float e) {
     // (e * 255 + 0.5).min(255) as u8: Rust's cast truncates and saturates (NaN -> 0)
     const float v = fminf(e * 255.0f + 0.5f, 255.0f);
     return v > 0.0f ? uint8_t(v) : uint8_t(0);
 }
 
-__global__ void k_to_rgb8(const float* __restrict__ hdr, uint32_t n, uint32_t tm, float white_point, float inv_gamma,
-                          float scale, uint8_t* __restrict__ out) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float c[3] = {hdr[3 * i] * scale, hdr[3 * i + 1] * scale, hdr[3 * i + 2] * scale};
-        float s = 1.0f;
+// The byte of a tone-mapped value m in [0, 1]: to_u8(powf(m, inv_gamma)).  powf
+// takes about a hundred instructions, and only decides the byte where e * 255 +
+// 0.5 lies next to an integer.  So the hardware logarithm and exponential (each
+// documented to 2^-22, absolute in (0.5, 2) for the logarithm, else relative) give
+// it first, and powf is called where their value lies within `guard` of an
+// integer.  With e |lg2 m| inv_gamma <= 1 / (e ln 2) they move e * 255 by at most
+// 6.7e-5 + 4.2e-5 inv_gamma; powf itself is within 4 ulp, 6e-5, and the last two
+// roundings within 3e-5.  The guard, 4e-4 max(1, inv_gamma), is twice the sum, so
+// every byte is powf's.
+__device__ __forceinline__ uint8_t encode_u8(float m, float inv_gamma, float guard) {
+    const float v = exp2f_approx(inv_gamma * log2f_approx(m)) * 255.0f + 0.5f;
+    if (fabsf(v - rintf(v)) > guard && (m >= FLT_MIN || m == 0.f)) return uint8_t(fminf(v, 255.0f));
+    return to_u8(powf(m, inv_gamma));
+}
+
+__device__ __forceinline__ void tone_map(float (&c)[3], uint32_t tm, float white_point, float scale) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) c[k] = c[k] * scale;
+    if (tm != AR_TONEMAP_CLAMP) {
+        const float lum = luminance(c[0], c[1], c[2]);
+        float s;
         if (tm == AR_TONEMAP_REINHARD) {
-            const float lum = luminance(c[0], c[1], c[2]);
             s = lum > 1e-6f ? (lum / (1.0f + lum)) / lum : 1.0f / (1.0f + lum);
-        } else if (tm == AR_TONEMAP_REINHARD_EXTENDED) {
+        } else {
             const float lw2 = white_point * white_point;
-            const float lum = luminance(c[0], c[1], c[2]);
             const float mapped = (lum * (1.0f + lum / lw2)) / (1.0f + lum);
             s = lum > 1e-6f ? mapped / lum : 1.0f;
         }
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            float m = tm == AR_TONEMAP_CLAMP ? c[k] : c[k] * s;
-            m = fminf(fmaxf(m, 0.0f), 1.0f);
-            out[3 * i + k] = to_u8(powf(m, inv_gamma));
+        for (int k = 0; k < 3; ++k) c[k] = c[k] * s;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) c[k] = fminf(fmaxf(c[k], 0.0f), 1.0f);
+}
+
+__device__ __forceinline__ void encode_pixel(const float* hdr, uint8_t* out, uint32_t tm, float white_point,
+                                             float inv_gamma, float guard, float scale) {
+    float c[3] = {hdr[0], hdr[1], hdr[2]};
+    tone_map(c, tm, white_point, scale);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) out[k] = encode_u8(c[k], inv_gamma, guard);
+}
+
+// kWide: four pixels a thread (three 16-byte loads, three 4-byte stores), the last
+// n % 4 one by one; where the addresses do not allow that, one pixel a thread.
+// 1921 x 1081, Reinhard extended: 26.3 -> 15.3 us with cold caches (the call
+// 69.8 -> 58.6).
+template <bool kWide>
+__global__ void __launch_bounds__(256) k_to_rgb8(const float* __restrict__ hdr, size_t n, uint32_t tm,
+                                                 float white_point, float inv_gamma, float guard, float scale,
+                                                 uint8_t* __restrict__ out) {
+    const size_t stride = size_t(gridDim.x) * blockDim.x, first = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    if constexpr (!kWide) {
+        for (size_t i = first; i < n; i += stride)
+            encode_pixel(hdr + 3 * i, out + 3 * i, tm, white_point, inv_gamma, guard, scale);
+    } else {
+        for (size_t j = first; j < (n + 3) / 4; j += stride) {
+            const size_t i = 4 * j;
+            if (i + 4 > n) {
+                for (size_t k = i; k < n; ++k)
+                    encode_pixel(hdr + 3 * k, out + 3 * k, tm, white_point, inv_gamma, guard, scale);
+                continue;
+            }
+            const float4* p = reinterpret_cast<const float4*>(hdr + 3 * i);
+            const float4 a = __ldcs(p), b = __ldcs(p + 1), c = __ldcs(p + 2);
+            const float v[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
+            uint32_t u[12];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float px[3] = {v[3 * q], v[3 * q + 1], v[3 * q + 2]};
+                tone_map(px, tm, white_point, scale);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) u[3 * q + k] = encode_u8(px[k], inv_gamma, guard);
+            }
+            uint32_t* o = reinterpret_cast<uint32_t*>(out + 3 * i);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) o[k] = u[4 * k] | u[4 * k + 1] << 8 | u[4 * k + 2] << 16 | u[4 * k + 3] << 24;
         }
     }
 }
@@ -242,8 +312,14 @@ void film_to_rgb8(ar_context* ctx, const float* hdr, uint32_t w, uint32_t h, uin
         AR_CUDA(cudaMemcpyAsync(d_hdr, hdr, n * 3 * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
         src = d_hdr;
     }
-    const int grid = std::max(1, std::min(int((n + 255) / 256), ctx->num_sms * 8));
-    k_to_rgb8<<<grid, 256, 0, ctx->stream>>>(src, uint32_t(n), tm, white_point, 1.0f / gamma, scale, dst);
+    const float inv_gamma = 1.0f / gamma, guard = 4e-4f * std::max(1.0f, inv_gamma);
+    const bool wide = reinterpret_cast<uintptr_t>(src) % 16 == 0 && reinterpret_cast<uintptr_t>(dst) % 4 == 0;
+    const size_t work = wide ? (n + 3) / 4 : n;
+    const int grid = int(std::max<size_t>(1, std::min<size_t>((work + 255) / 256, size_t(ctx->num_sms) * 8)));
+    if (wide)
+        k_to_rgb8<true><<<grid, 256, 0, ctx->stream>>>(src, n, tm, white_point, inv_gamma, guard, scale, dst);
+    else
+        k_to_rgb8<false><<<grid, 256, 0, ctx->stream>>>(src, n, tm, white_point, inv_gamma, guard, scale, dst);
     AR_CUDA(cudaGetLastError());
     if (!on_device) {
         AR_CUDA(cudaMemcpyAsync(out, dst, n * 3, cudaMemcpyDeviceToHost, ctx->stream));

@@ -125,3 +125,25 @@ def test_cg_sizes_reach_the_exact_solution(ctx, h, w):
     b = np.linalg.norm((0.2 * primal.astype(np.float64) + div).reshape(-1, 3), axis=0)
     want = np.maximum(exact, 0)
     assert np.all(np.abs(out - want) <= 5e-6 * b + 2e-7 * np.abs(want))
+
+
+@pytest.mark.parametrize("h,w", [(1, 1), (1, 3), (1, 4), (7, 5), (33, 31)])
+@pytest.mark.parametrize("tm,gamma", [(A.TONEMAP_CLAMP, 2.2), (A.TONEMAP_REINHARD, 1.0),
+                                      (A.TONEMAP_REINHARD_EXTENDED, 0.5)])
+def test_rgb8_does_not_depend_on_size_or_alignment(ctx, h, w, tm, gamma):
+    # Whole quads, their tails, and images whose address is not 16-byte aligned
+    # (one pixel a thread) give the same bytes, at most 1 LSB from the oracle's
+    # libm powf on the few values next to a rounding boundary.
+    import torch
+    import oracle as O
+    rng = np.random.default_rng(h * 100 + w)
+    hdr = rng.lognormal(-1.0, 1.5, (h, w, 3)).astype(np.float32)
+    flat = hdr.reshape(-1)
+    flat[:3] = [0.0, -1.0, 1.0]
+    dev = torch.from_numpy(hdr).cuda()
+    want = agentray.film_to_rgb8(ctx, dev, tm, gamma, 1.5, 4.0).cpu().numpy()
+    shifted = torch.zeros(h * w * 3 + 1, device="cuda")[1:].view(h, w, 3)
+    shifted.copy_(dev)
+    np.testing.assert_array_equal(agentray.film_to_rgb8(ctx, shifted, tm, gamma, 1.5, 4.0).cpu().numpy(), want)
+    d = np.abs(want.astype(int) - O.film_to_rgb8(hdr, tm, 4.0, gamma, 1.5).astype(int))
+    assert d.max() <= 1 and (d > 0).sum() <= max(1, 1e-3 * d.size)

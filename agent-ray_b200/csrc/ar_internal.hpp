@@ -147,6 +147,7 @@ struct ar_context {
     ar::Workspace solver;     // Poisson solver buffers
     ar::Profiler prof;
     uint64_t* stats_h = nullptr;  // pinned copy of stats_d, valid after a sync
+    int* flag_h = nullptr;        // pinned copy of err_flag
     ar_render_stats last_stats{};
     bool stats_pending = false;
     ar::PathEngine* engine = nullptr;  // streaming wavefront engine for ar_render

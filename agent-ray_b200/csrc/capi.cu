@@ -22,9 +22,10 @@ void launch_trace(ar_context* ctx, const ar_scene* sc, const float4* ot, const f
 
 // Checks the device error flag after a synchronisation.
 void check_device_flag(ar_context* ctx) {
-    int flag = 0;
-    AR_CUDA(cudaMemcpyAsync(&flag, ctx->err_flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    // into pinned memory: the copy is queued behind the stream's work, and one wait covers both
+    AR_CUDA(cudaMemcpyAsync(ctx->flag_h, ctx->err_flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     AR_CUDA(cudaStreamSynchronize(ctx->stream));
+    const int flag = *ctx->flag_h;
     if (flag) {
         AR_CUDA(cudaMemsetAsync(ctx->err_flag.ptr, 0, sizeof(int), ctx->stream));
         AR_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -52,6 +53,7 @@ ar_context* context_create_internal(int device) {
     ctx->stats_d.alloc(8 * sizeof(uint64_t));
     AR_CUDA(cudaMemset(ctx->stats_d.ptr, 0, 8 * sizeof(uint64_t)));
     AR_CUDA(cudaMallocHost(&ctx->stats_h, 8 * sizeof(uint64_t)));
+    AR_CUDA(cudaMallocHost(&ctx->flag_h, sizeof(int)));
     std::memset(ctx->stats_h, 0, 8 * sizeof(uint64_t));
     return ctx.release();
 }
@@ -78,6 +80,7 @@ void context_destroy_internal(ar_context* ctx) {
     if (ctx->copy_out) cudaStreamDestroy(ctx->copy_out);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     if (ctx->stats_h) cudaFreeHost(ctx->stats_h);
+    if (ctx->flag_h) cudaFreeHost(ctx->flag_h);
     delete ctx;
 }
 
@@ -112,8 +115,7 @@ int ar_context_set_stream(ar_context* ctx, void* stream) {
 int ar_context_synchronize(ar_context* ctx) {
     return guarded([&] {
         AR_REQUIRE(ctx, AR_ERR_INVALID_ARGUMENT, "ctx is null");
-        AR_CUDA(cudaStreamSynchronize(ctx->stream));
-        check_device_flag(ctx);
+        check_device_flag(ctx);  // waits for the stream
     });
 }
 

@@ -12,18 +12,19 @@ constexpr uint32_t kMaxBdptJobs = 1024;
 struct alignas(16) BdJob {
     DevScene sc;
     CameraDev cam;
-    uint32_t width, height, spp, max_depth, rr_depth, mis_mode;
+    uint32_t width, height, samples, max_depth, rr_depth, mis_mode;  // samples: per pixel, from first_sample
     float mis_beta;
     uint32_t film64;
     uint64_t seed;
     float inv_spp;
-    float pad;
+    uint32_t first_sample;
     void* film;
 };
 
 // Batch samples [offset, offset + nsamples) are samples
 // [sample_begin, sample_begin + nsamples) of job `job` (index into the
-// batch's job list).  Segments are sorted by offset and contiguous.
+// batch's job list), number g being pixel g / samples, sample g % samples.
+// Segments are sorted by offset and contiguous.
 struct BdSegment {
     uint32_t job, offset, nsamples, pad;
     unsigned long long sample_begin;

@@ -32,12 +32,12 @@ constexpr uint32_t kEngineTickKernels = 5;
 struct alignas(16) JobDev {
     DevScene sc;
     CameraDev cam;
-    uint32_t width, height, spp, max_depth, rr_depth, gdpt, film64, roles;
+    uint32_t width, height, samples, max_depth, rr_depth, gdpt, film64, roles;  // samples: per pixel, from first_sample
     uint64_t seed;
     float inv_spp;
-    float pad0;
+    uint32_t first_sample;
     void* film[3];
-    unsigned long long total_samples;  // W*H*spp
+    unsigned long long total_samples;  // W*H*samples; number g is pixel g / samples, sample g % samples
     unsigned long long next_sample;    // generation cursor (advanced by the plan kernel)
     unsigned long long total_paths;    // samples * roles
     unsigned long long done_paths;     // finished (deposited) paths

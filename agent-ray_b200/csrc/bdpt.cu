@@ -48,7 +48,7 @@ struct BdParams {
     uint32_t cap;         // batch capacity: the stride of the per-sample arrays
     uint32_t maxv;        // vertex capacity per subpath
     uint32_t* sjob;     // job of each batch sample
-    unsigned long long* sindex;  // global sample index of each batch sample
+    uint2* spix;        // pixel and sample of each batch sample
     float4* va;  // p.xyz, pdf_fwd
     float4* vb;  // n.xyz, pdf_rev
     float4* vc;  // thr.xyz, info (type << 30 | delta << 29 | index)
@@ -265,12 +265,12 @@ __global__ void __launch_bounds__(256) k_bd_generate(BdParams P) {
             const BdSegment sg = P.seg[lo];
             const BdJob& J = P.jobs[sg.job];
             const unsigned long long g = sg.sample_begin + (si - sg.offset);
-            const uint32_t npix = J.width * J.height;
-            const uint32_t pixel = uint32_t(g % npix), sample = uint32_t(g / npix);
+            // all samples of a pixel together, as the path engine generates them
+            const uint32_t pixel = uint32_t(g / J.samples), sample = J.first_sample + uint32_t(g % J.samples);
             const uint64_t key = counter_key(J.seed, pixel, sample);
             if (sub == 0) {
                 P.sjob[si] = sg.job;
-                P.sindex[si] = g;
+                P.spix[si] = make_uint2(pixel, sample);
                 const float jx = counter_u01(key, 0), jy = counter_u01(key, 1);
                 const uint32_t px = pixel % J.width, py = pixel / J.width;
                 r = camera_ray(J.cam, (float(px) + jx) / float(J.width), 1.0f - (float(py) + jy) / float(J.height));
@@ -380,9 +380,8 @@ __global__ void __launch_bounds__(256, 4) k_bd_vertex(BdParams P, uint32_t depth
                 store_vtx(P, sub, k, si, s.p, s.n, thr, pdf_fwd, kTypeSurface, false, s.mat,
                           J.sc.materials[s.mat].tex >= 0, s.tu, s.tv);
                 P.nv[sub * P.cap + si] = uint8_t(k + 1);
-                const unsigned long long g = P.sindex[si];
-                const uint32_t npix = J.width * J.height;
-                const uint64_t key = counter_key(J.seed, uint32_t(g % npix), uint32_t(g / npix));
+                const uint2 ps = P.spix[si];
+                const uint64_t key = counter_key(J.seed, ps.x, ps.y);
                 uint32_t d = P.dim[spi];
                 const f3 wo_l = to_local(s.onb, -rd);
                 const float usel = counter_u01(key, d++);
@@ -778,7 +777,7 @@ __global__ void __launch_bounds__(kConnectThreads, kConnectBlocks) k_bd_connect(
                 const BdJob& J = P.jobs[job];
                 S = P.nv[si];
                 T = P.nv[P.cap + si];
-                pix = uint32_t(P.sindex[si] % (J.width * J.height));
+                pix = P.spix[si].x;
                 if (J.mis_mode == AR_MIS_POWER && J.mis_beta == 2.0f && S <= kMisCache && T <= kMisCache)
                     flags |= kFlagFastMis;
                 if (T >= 1 && J.sc.lights[load_vtx(P, 1, 0, si).index].kind == AR_LIGHT_POINT) flags |= kFlagPointLight;
@@ -946,7 +945,7 @@ BdptBatcher* bdpt_create(ar_context* ctx, uint32_t max_depth_cap, uint32_t batch
     P.hit = carve<float4>(cur, 2 * size_t(batch));
     P.hit_inst = carve<uint32_t>(cur, 2 * size_t(batch));
     P.sjob = carve<uint32_t>(cur, batch);
-    P.sindex = carve<unsigned long long>(cur, batch);
+    P.spix = carve<uint2>(cur, batch);
     P.sh_cap = uint32_t(std::min<uint64_t>(uint64_t(max_pairs_for(max_depth_cap)) * batch, 0xFFFFFFF0ull));
     P.sh_o = carve<float4>(cur, P.sh_cap);
     P.sh_d = carve<float4>(cur, P.sh_cap);
@@ -1080,7 +1079,7 @@ BdJob make_bdpt_job(const ar_scene* sc, const CameraDev& cam, const ar_integrato
     J.cam = cam;
     J.width = w;
     J.height = h;
-    J.spp = cfg.spp;
+    J.samples = cfg.spp;
     J.max_depth = cfg.max_depth;
     J.rr_depth = cfg.rr_depth;
     J.mis_mode = cfg.mis_mode;
@@ -1098,7 +1097,7 @@ void render_bdpt_film(ar_context* ctx, const ar_scene* sc, const CameraDev& cam,
     AR_REQUIRE(cfg.max_depth <= 62, AR_ERR_INVALID_ARGUMENT, "max_depth must be <= 62");
     const uint64_t npix = uint64_t(w) * h;
     const uint32_t s0 = ctx->range_end ? ctx->range_begin : 0u, s1 = ctx->range_end ? ctx->range_end : cfg.spp;
-    const uint64_t first = npix * s0, total = npix * (s1 - s0);
+    const uint64_t total = npix * (s1 - s0);
     const size_t budget = ctx->bdpt_budget;
     const size_t per = bdpt_batch_bytes(cfg.max_depth, 1024) / 1024 + 1;
     const uint64_t fit = std::max<uint64_t>(1024, budget / per);
@@ -1138,14 +1137,16 @@ void render_bdpt_film(ar_context* ctx, const ar_scene* sc, const CameraDev& cam,
         AR_CUDA(cudaEventRecord(ctx->lane_ev[0], ctx->stream));
         AR_CUDA(cudaStreamWaitEvent(ctx->lane_stream, ctx->lane_ev[0], 0));
     }
-    const std::vector<BdJob> jobs{make_bdpt_job(sc, cam, cfg, w, h, film)};
+    std::vector<BdJob> jobs{make_bdpt_job(sc, cam, cfg, w, h, film)};
+    jobs[0].first_sample = s0;
+    jobs[0].samples = s1 - s0;
     uint64_t batches = 0;
     for (uint64_t begin = 0; begin < total; begin += cap, ++batches) {
         const uint32_t n = uint32_t(std::min<uint64_t>(cap, total - begin));
         if (two_lanes && (batches & 1))
-            bdpt_run_batch(ctx->bdpt2, jobs, {BdSegment{0, 0, n, 0, first + begin}}, ctx->lane_stream);
+            bdpt_run_batch(ctx->bdpt2, jobs, {BdSegment{0, 0, n, 0, begin}}, ctx->lane_stream);
         else
-            bdpt_run_batch(ctx->bdpt, jobs, {BdSegment{0, 0, n, 0, first + begin}});
+            bdpt_run_batch(ctx->bdpt, jobs, {BdSegment{0, 0, n, 0, begin}});
     }
     if (two_lanes) {  // join: the context stream waits for the second lane
         AR_CUDA(cudaEventRecord(ctx->lane_ev[1], ctx->lane_stream));

@@ -176,8 +176,12 @@ __global__ void __launch_bounds__(256) k_generate(EngineDev E, int q) {
         const uint32_t rel = k - sg.path_offset;
         const uint32_t si = rel / sg.roles, role = rel - si * sg.roles;
         const unsigned long long g = sg.sample_begin + si;
-        const uint32_t npix = J.width * J.height;
-        const uint32_t pixel = uint32_t(g % npix), sample = uint32_t(g / npix);
+        // all samples of a pixel together, pixels row by row: a warp's camera rays
+        // and what they first hit stay together (against one sample of every pixel
+        // after the other: extension -7%, render -4.5% at 512x512x16 on 139k
+        // triangles; 32x32 blocks in Z order instead of rows gave 0.2% more, 8x4
+        // tiles of one sample each 1.4%)
+        const uint32_t pixel = uint32_t(g / J.samples), sample = J.first_sample + uint32_t(g % J.samples);
         const uint32_t px = pixel % J.width, py = pixel / J.width;
         const bool skip = (role == kRoleRight && px + 1 >= J.width) || (role == kRoleDown && py + 1 >= J.height);
         if (skip) {
@@ -650,7 +654,6 @@ void render_pt_films(ar_context* ctx, const ar_scene* sc, const CameraDev& cam, 
     J.cam = cam;
     J.width = w;
     J.height = h;
-    J.spp = cfg.spp;
     J.max_depth = cfg.max_depth;
     J.rr_depth = cfg.rr_depth;
     J.gdpt = gdpt ? 1u : 0u;
@@ -661,9 +664,11 @@ void render_pt_films(ar_context* ctx, const ar_scene* sc, const CameraDev& cam, 
     for (uint32_t f = 0; f < roles; ++f) J.film[f] = static_cast<char*>(films) + f * film_bytes;
     const uint64_t npix = uint64_t(w) * h;
     const uint32_t s0 = ctx->range_end ? ctx->range_begin : 0u, s1 = ctx->range_end ? ctx->range_end : cfg.spp;
-    J.total_samples = npix * s1;  // sample g of the job is pixel g % npix, sample g / npix
+    J.samples = s1 - s0;
+    J.first_sample = s0;
+    J.total_samples = npix * (s1 - s0);
     J.total_paths = npix * (s1 - s0) * roles;
-    J.next_sample = npix * s0;
+    J.next_sample = 0;
     J.done_paths = 0;
     const uint32_t slot = 0;
     engine_add_job(e, slot, J);

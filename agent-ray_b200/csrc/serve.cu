@@ -246,7 +246,7 @@ struct ServerImpl {
                 J.cam = cam;
                 J.width = j->w;
                 J.height = j->h;
-                J.spp = j->cfg.spp;
+                J.samples = j->cfg.spp;
                 J.max_depth = j->cfg.max_depth;
                 J.rr_depth = j->cfg.rr_depth;
                 J.gdpt = nf == 3 ? 1u : 0u;

@@ -140,7 +140,7 @@ __device__ __forceinline__ TriRecord load_tri(const TriRecord* rec) {
     float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
     TriRecord r;
     r.v0x = a.x; r.v0y = a.y; r.v0z = a.z; r.prim = __float_as_uint(a.w);
-    r.e1x = b.x; r.e1y = b.y; r.e1z = b.z; r.object_local = __float_as_uint(b.w);
+    r.e1x = b.x; r.e1y = b.y; r.e1z = b.z; r.mesh = __float_as_uint(b.w);
     r.e2x = c.x; r.e2y = c.y; r.e2z = c.z; r.slot = __float_as_uint(c.w);
     return r;
 }

@@ -185,7 +185,7 @@ struct ar_scene {
     std::vector<std::vector<uint32_t>> object_mats;
     std::vector<float> light_power_weights;
     // device data
-    ar::DevBuf geom, objects_d, meshes_d, indices, normals, slots, mat_table, materials, lights,
+    ar::DevBuf geom, shade, objects_d, meshes_d, indices, normals, slots, mat_table, materials, lights,
         light_cdf, light_pmf, texcoords, texels, textures;
     ar::DevScene view{};
     ar_scene_stats stats{};

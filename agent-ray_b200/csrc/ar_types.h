@@ -41,7 +41,7 @@ struct alignas(16) TriRecord {
     float v0x, v0y, v0z;
     uint32_t prim;
     float e1x, e1y, e1z;
-    uint32_t object_local;  // unused padding
+    uint32_t mesh;
     float e2x, e2y, e2z;
     uint32_t slot;  // this record's index
 };
@@ -62,7 +62,22 @@ struct alignas(16) ObjectRecord {
     uint32_t mesh;
     uint32_t mat_offset;  // into material_table
     uint32_t num_mats;
+    uint32_t flags;       // kMeshNormals, kMeshUv
+    uint32_t mat0;        // the first material (the material, when there is one)
+    uint32_t pad[2];
 };
+static_assert(sizeof(ObjectRecord) == 64, "object record is 64 bytes");
+constexpr uint32_t kMeshNormals = 1u, kMeshUv = 2u;
+
+// What shading reads of a triangle beside its TriRecord, gathered when the
+// acceleration structure is built: its vertices' normals and uv and its material
+// slot.
+struct alignas(16) TriShade {
+    float n[9];     // normals of the three vertices
+    uint32_t slot;  // material slot
+    float uv[6];
+};
+static_assert(sizeof(TriShade) == 64, "shading record is 64 bytes");
 
 struct alignas(16) MeshRecord {
     uint32_t idx_offset;   // into indices (3 per triangle, original order)
@@ -102,17 +117,13 @@ struct alignas(16) LightRecord {
 struct DevScene {
     const WideNode* nodes;  // nodes, triangle and instance records in one buffer
     const TriRecord* tris;  // the triangle records of that buffer
+    const TriShade* shade;  // per triangle record
     const ObjectRecord* objects;
-    const MeshRecord* meshes;
-    const uint32_t* indices;
-    const float* normals;
-    const uint32_t* material_slots;
     const uint32_t* material_table;
     const MaterialRecord* materials;
     const LightRecord* lights;
     const float* light_cdf;
     const float* light_pmf;
-    const float* texcoords;
     const float4* texels;
     const TextureRecord* textures;
     uint32_t tlas_root;       // 0xFFFFFFFF: empty scene

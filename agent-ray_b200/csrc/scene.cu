@@ -42,6 +42,25 @@ void upload(DevBuf& d, const std::vector<T>& h) {
     if (!h.empty()) AR_CUDA(cudaMemcpy(d.ptr, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
 }
 
+// TriShade of every triangle record (of its mesh).
+__global__ void k_gather_shade(const TriRecord* tris, uint32_t n, const MeshRecord* meshes, const uint32_t* indices,
+                               const float* normals, const float* texcoords, const uint32_t* slots, TriShade* out) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t prim = tris[i].prim;
+        const MeshRecord m = meshes[tris[i].mesh];
+        const uint32_t* ix = indices + m.idx_offset + 3 * size_t(prim);
+        TriShade t{};
+        for (int k = 0; k < 3; ++k) {
+            if (m.nrm_offset != kInvalid)
+                for (int j = 0; j < 3; ++j) t.n[3 * k + j] = normals[3 * (size_t(m.nrm_offset) + ix[k]) + j];
+            if (m.uv_offset != kInvalid)
+                for (int j = 0; j < 2; ++j) t.uv[2 * k + j] = texcoords[2 * (size_t(m.uv_offset) + ix[k]) + j];
+        }
+        t.slot = m.num_slots == 1 ? slots[m.slot_offset] : slots[m.slot_offset + prim];
+        out[i] = t;
+    }
+}
+
 struct V3f {
     float x, y, z;
 };
@@ -136,7 +155,7 @@ void build_scene_accel(ar_scene* s, const ar_accel_opts* o) {
             tr.prim = p;
             tr.e1x = v1[0] - v0[0]; tr.e1y = v1[1] - v0[1]; tr.e1z = v1[2] - v0[2];
             tr.e2x = v2[0] - v0[0]; tr.e2y = v2[1] - v0[1]; tr.e2z = v2[2] - v0[2];
-            tr.object_local = uint32_t(m);
+            tr.mesh = uint32_t(m);
             tr.slot = uint32_t(tris.size());
             tris.push_back(tr);
             for (int k = 0; k < 3; ++k) {
@@ -229,6 +248,17 @@ void build_scene_accel(ar_scene* s, const ar_accel_opts* o) {
     s->view.nodes = s->geom.as<WideNode>();
     s->view.tris = reinterpret_cast<const TriRecord*>(geom + tri_word);
     s->view.tlas_root = tlas_root;
+    // the triangles' shading records, gathered on the device from the uploaded arrays
+    s->shade.alloc(std::max<size_t>(1, tris.size()) * sizeof(TriShade));
+    s->view.shade = s->shade.as<TriShade>();
+    if (!tris.empty()) {
+        const int grid = int(std::min<size_t>((tris.size() + 255) / 256, 4096));
+        k_gather_shade<<<grid, 256>>>(s->view.tris, uint32_t(tris.size()), s->meshes_d.as<MeshRecord>(),
+                                      s->indices.as<uint32_t>(), s->normals.as<float>(), s->texcoords.as<float>(),
+                                      s->slots.as<uint32_t>(), s->shade.as<TriShade>());
+        AR_CUDA(cudaGetLastError());
+        AR_CUDA(cudaStreamSynchronize(nullptr));
+    }
     s->stats.num_blas_nodes = blas_nodes;
     s->stats.num_tlas_nodes = tlas_nodes;
     s->stats.num_instances = inst_rec.size();
@@ -314,6 +344,9 @@ void create_scene(ar_context* ctx, const ar_scene_desc* d, ar_scene** out) {
         orec[i].mesh = od.mesh;
         orec[i].mat_offset = uint32_t(mat_table.size());
         orec[i].num_mats = od.num_materials;
+        orec[i].flags = (mrec[od.mesh].nrm_offset != kInvalid ? kMeshNormals : 0u) |
+                        (mrec[od.mesh].uv_offset != kInvalid ? kMeshUv : 0u);
+        orec[i].mat0 = od.materials[0];
         mat_table.insert(mat_table.end(), od.materials, od.materials + od.num_materials);
     }
     // materials
@@ -415,13 +448,8 @@ void create_scene(ar_context* ctx, const ar_scene_desc* d, ar_scene** out) {
     upload(s->light_cdf, s->cdf_h);
     upload(s->light_pmf, s->pmf_h);
     s->view.objects = s->objects_d.as<ObjectRecord>();
-    s->view.meshes = s->meshes_d.as<MeshRecord>();
-    s->view.indices = s->indices.as<uint32_t>();
-    s->view.normals = s->normals.as<float>();
-    s->view.texcoords = s->texcoords.as<float>();
     s->view.texels = s->texels.as<float4>();
     s->view.textures = s->textures.as<TextureRecord>();
-    s->view.material_slots = s->slots.as<uint32_t>();
     s->view.material_table = s->mat_table.as<uint32_t>();
     s->view.materials = s->materials.as<MaterialRecord>();
     s->view.lights = s->lights.as<LightRecord>();
@@ -432,7 +460,7 @@ void create_scene(ar_context* ctx, const ar_scene_desc* d, ar_scene** out) {
     s->stats.num_triangles = ntri_total;
     build_scene_accel(s.get(), nullptr);
     size_t bytes = 0;
-    for (DevBuf* b : {&s->geom, &s->objects_d, &s->meshes_d, &s->indices, &s->normals,
+    for (DevBuf* b : {&s->geom, &s->shade, &s->objects_d, &s->meshes_d, &s->indices, &s->normals,
                       &s->slots, &s->mat_table, &s->materials, &s->lights, &s->light_cdf, &s->light_pmf,
                       &s->texcoords, &s->texels, &s->textures})
         bytes += b->bytes;

@@ -348,8 +348,53 @@ __global__ void AR_TRAVERSAL_BOUNDS k_bd_extend(const __grid_constant__ BdParams
         });
 }
 
-// One bounce of both subpaths (:368-434, :498-556).  <= 64 registers, as
-// k_shade: latency-bound, faster at double occupancy despite spills.
+// One bounce of a subpath (:368-434, :498-556): appends the hit's vertex to
+// subpath q, sets the previous vertex's pdf_rev and samples the next ray.
+// Returns whether the subpath goes on (with the ray no, nd).
+__device__ __forceinline__ bool bd_vertex(const BdParams& P, const BdJob& J, uint32_t q, uint32_t depth, f3 ro, f3 rd,
+                                          float ht, float hu, float hv, uint32_t slot, uint32_t inst, f3& no, f3& nd) {
+    const uint32_t si = q >> 1, sub = q & 1u;
+    const Shade s = make_shade(J.sc, ro, rd, ht, hu, hv, slot, inst);
+    const MatView m = load_mat_at(J.sc, s.mat, s.tu, s.tv);
+    const uint32_t spi = sp_slot(P, q);
+    const float4 t4 = P.thr[spi];
+    f3 thr = mk(t4.x, t4.y, t4.z);
+    const uint32_t k = P.nv[sub * P.cap + si];  // index of the new vertex
+    const size_t pi = vidx(P, sub, k - 1, si);
+    const float4 pa = P.va[pi], pb = P.vb[pi];
+    const f3 prev_p = mk(pa.x, pa.y, pa.z), prev_n = mk(pb.x, pb.y, pb.z);
+    const float pdf_fwd = pdf_sa_to_area(t4.w, prev_p, s.p, s.n);
+    store_vtx(P, sub, k, si, s.p, s.n, thr, pdf_fwd, kTypeSurface, false, s.mat, J.sc.materials[s.mat].tex >= 0, s.tu,
+              s.tv);
+    P.nv[sub * P.cap + si] = uint8_t(k + 1);
+    const uint2 ps = P.spix[si];
+    const uint64_t key = counter_key(J.seed, ps.x, ps.y);
+    uint32_t d = P.dim[spi];
+    const f3 wo_l = to_local(s.onb, -rd);
+    const float usel = counter_u01(key, d++);
+    const float ux = counter_u01(key, d++), uy = counter_u01(key, d++);
+    f3 wi, f;
+    float pdf;
+    if (!(bsdf_sample(m, wo_l, usel, ux, uy, wi, pdf, f) && pdf != 0.f && !is_zero(f))) return false;
+    thr = thr * ((f * fabsf(wi.z)) / pdf);
+    const float pdf_rev_dir = bsdf_pdf(m, wo_l, wi);
+    P.vb[pi].w = pdf_sa_to_area(pdf_rev_dir, s.p, prev_p, prev_n);
+    if (depth + 1 >= J.rr_depth) {
+        const float survival = fminf(max3(thr), 0.95f);
+        if (counter_u01(key, d++) > survival || survival <= 0.f) return false;
+        thr = thr / survival;
+    }
+    if (depth + 1 >= J.max_depth) return false;
+    const f3 wi_w = to_world(s.onb, wi);
+    no = s.p + (s.n * 1e-4f) * signum(dot(wi_w, s.n));
+    nd = normalize(wi_w);
+    P.thr[spi] = make_float4(thr.x, thr.y, thr.z, pdf);
+    P.dim[spi] = d;
+    return true;
+}
+
+// <= 64 registers, as k_shade: latency-bound, faster at double occupancy
+// despite spills.
 __global__ void __launch_bounds__(256, 4) k_bd_vertex(BdParams P, uint32_t depth) {
     const uint32_t n = P.counts[depth];
     const int b = depth & 1;
@@ -360,53 +405,13 @@ __global__ void __launch_bounds__(256, 4) k_bd_vertex(BdParams P, uint32_t depth
         f3 no, nd;
         if (j < n) {
             q = P.qpath[b][j];
-            const uint32_t si = q >> 1, sub = q & 1u;
-            const BdJob& J = P.jobs[P.sjob[si]];
+            const BdJob& J = P.jobs[P.sjob[q >> 1]];
             const float4 h = P.hit[j];
             const uint32_t slot = __float_as_uint(h.w);
             if (slot != kInvalid) {
                 const float4 ro4 = P.ray_o[b][j], rd4 = P.ray_d[b][j];
-                const f3 ro = mk(ro4.x, ro4.y, ro4.z), rd = mk(rd4.x, rd4.y, rd4.z);
-                const Shade s = make_shade(J.sc, ro, rd, h.x, h.y, h.z, slot, P.hit_inst[j]);
-                const MatView m = load_mat_at(J.sc, s.mat, s.tu, s.tv);
-                const uint32_t spi = sp_slot(P, q);
-                const float4 t4 = P.thr[spi];
-                f3 thr = mk(t4.x, t4.y, t4.z);
-                const uint32_t k = P.nv[sub * P.cap + si];  // index of the new vertex
-                const size_t pi = vidx(P, sub, k - 1, si);
-                const float4 pa = P.va[pi], pb = P.vb[pi];
-                const f3 prev_p = mk(pa.x, pa.y, pa.z), prev_n = mk(pb.x, pb.y, pb.z);
-                const float pdf_fwd = pdf_sa_to_area(t4.w, prev_p, s.p, s.n);
-                store_vtx(P, sub, k, si, s.p, s.n, thr, pdf_fwd, kTypeSurface, false, s.mat,
-                          J.sc.materials[s.mat].tex >= 0, s.tu, s.tv);
-                P.nv[sub * P.cap + si] = uint8_t(k + 1);
-                const uint2 ps = P.spix[si];
-                const uint64_t key = counter_key(J.seed, ps.x, ps.y);
-                uint32_t d = P.dim[spi];
-                const f3 wo_l = to_local(s.onb, -rd);
-                const float usel = counter_u01(key, d++);
-                const float ux = counter_u01(key, d++), uy = counter_u01(key, d++);
-                f3 wi, f;
-                float pdf;
-                if (bsdf_sample(m, wo_l, usel, ux, uy, wi, pdf, f) && pdf != 0.f && !is_zero(f)) {
-                    thr = thr * ((f * fabsf(wi.z)) / pdf);
-                    const float pdf_rev_dir = bsdf_pdf(m, wo_l, wi);
-                    P.vb[pi].w = pdf_sa_to_area(pdf_rev_dir, s.p, prev_p, prev_n);
-                    bool alive = true;
-                    if (depth + 1 >= J.rr_depth) {
-                        const float survival = fminf(max3(thr), 0.95f);
-                        if (counter_u01(key, d++) > survival || survival <= 0.f) alive = false;
-                        else thr = thr / survival;
-                    }
-                    if (alive && depth + 1 < J.max_depth) {
-                        const f3 wi_w = to_world(s.onb, wi);
-                        no = s.p + (s.n * 1e-4f) * signum(dot(wi_w, s.n));
-                        nd = normalize(wi_w);
-                        P.thr[spi] = make_float4(thr.x, thr.y, thr.z, pdf);
-                        P.dim[spi] = d;
-                        cont = true;
-                    }
-                }
+                cont = bd_vertex(P, J, q, depth, mk(ro4.x, ro4.y, ro4.z), mk(rd4.x, rd4.y, rd4.z), h.x, h.y, h.z, slot,
+                                 P.hit_inst[j], no, nd);
             }
         }
         const uint32_t rs = warp_alloc(&P.counts[depth + 1], cont);
@@ -415,6 +420,78 @@ __global__ void __launch_bounds__(256, 4) k_bd_vertex(BdParams P, uint32_t depth
             P.ray_d[b ^ 1][rs] = make_float4(nd.x, nd.y, nd.z, FLT_MAX);
             P.qpath[b ^ 1][rs] = q;
         }
+    }
+}
+
+// Both subpaths of a small batch, all bounces in one launch.  A stage of few rays
+// takes as long as its longest ray (about 70 us for 100,000 rays of a small scene,
+// three times the mean), and a batch is max_depth such stages one after the
+// other; here a warp goes on to its next bounce when its own rays are done.
+// The same work in the same order for every subpath, so the same vertices.
+// Up to 1.5 samples (3 subpaths) a lane of the grid, where the two forms meet:
+// 16k, 65k, 131k, 262k samples of a small scene 700 -> 566 us, 1151 -> 999, 1750 ->
+// 1724, 2947 -> 3178; of the 195k-triangle room 945 -> 769, 1502 -> 1232, 2149 ->
+// 2033, 3444 -> 3648 (stages -> this, whole render).  5 blocks per SM (96 registers):
+// 4, 6 and 8 gave 1010, 1023 and 1093 us at 65k; going on as soon as half or a
+// quarter of a warp's rays are done 1115 and 1024.
+constexpr uint32_t kWalkBlocks = 5;
+bool use_walk(uint32_t samples, int num_sms) { return uint64_t(samples) * 2 <= 3ull * num_sms * kWalkBlocks * 128; }
+
+__global__ void __launch_bounds__(128, kWalkBlocks) k_bd_walk(const __grid_constant__ BdParams P, int* err) {
+    const uint32_t n = P.counts[0], lane = threadIdx.x & 31u;
+    Traverser<false> tr;
+    uint2 mem[Traverser<false>::kSlots];
+    uint32_t q = kInvalid, depth = 0;  // this lane's subpath, kInvalid: none
+    f3 ro, rd;
+    float tmin = 0.f, tmax = 0.f;
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    bool more = lane < (n < 5u * warps ? (n + n / 2u + warps - 1u) / warps : 32u);
+    for (;;) {
+        const bool need = more && q == kInvalid;
+        const uint32_t j = warp_alloc(&P.counts[kBdExtendCursor], need);
+        if (need) {
+            more = j < n;
+            if (more) {
+                const float4 a = P.ray_o[0][j], d = P.ray_d[0][j];
+                q = P.qpath[0][j];
+                ro = mk(a.x, a.y, a.z);
+                rd = mk(d.x, d.y, d.z);
+                tmin = a.w;
+                tmax = d.w;
+                depth = 0;
+            }
+        }
+        if (!__any_sync(0xffffffffu, q != kInvalid)) break;
+        const BdJob* J = nullptr;
+        bool busy = false;
+        if (q != kInvalid) {
+            J = &P.jobs[P.sjob[q >> 1]];
+            busy = tr.start(&J->sc, Ray{ro, rd, tmin, tmax}, mem);
+        }
+        while (__any_sync(0xffffffffu, busy)) {
+            if (busy) {
+#pragma unroll 1
+                for (int k = 0; k < kStepsClosest && busy; ++k) busy = !tr.step(err, mem);
+            }
+        }
+        bool cont = false;
+        if (q != kInvalid) {
+            const HitRec h = tr.result(mem);
+            f3 no, nd;
+            cont = h.slot != kInvalid && bd_vertex(P, *J, q, depth, ro, rd, h.t, h.u, h.v, h.slot, h.inst, no, nd);
+            if (cont) {
+                ro = no;
+                rd = nd;
+                tmin = 1e-4f;
+                tmax = FLT_MAX;
+                depth++;
+            } else {
+                q = kInvalid;
+            }
+        }
+        // rays per bounce, as the stages count them
+        const uint32_t same = __match_any_sync(0xffffffffu, cont ? depth : kInvalid);
+        if (cont && int(lane) == __ffs(same) - 1) atomicAdd(&P.counts[depth], uint32_t(__popc(same)));
     }
 }
 
@@ -899,7 +976,7 @@ struct BdptBatcher {
     // The stage sequence of a batch captured as one CUDA graph per max depth
     // (the kernels read the batch's size from dyn_d, so a graph serves every
     // batch of that depth), replayed on captured_stream.
-    cudaGraphExec_t graphs[63] = {};
+    cudaGraphExec_t graphs[2 * 63] = {};
     cudaStream_t captured_stream = nullptr;
 };
 
@@ -975,10 +1052,16 @@ void bdpt_destroy(BdptBatcher* b) {
 uint32_t bdpt_batch_capacity(const BdptBatcher* b) { return b->batch; }
 uint32_t bdpt_max_depth_cap(const BdptBatcher* b) { return b->max_depth_cap; }
 
+// generate, walk or (extend, vertex) per depth, hist/scan/scatter, connect,
+// shadow, count
+static uint32_t batch_kernels(uint32_t max_depth, bool walk) {
+    return (walk ? (max_depth ? 1 : 0) : 2 * max_depth) + 7;
+}
+
 // The stages of one batch whose jobs reach `max_depth` bounces, on stream
 // `s`; grids are sized for the batch capacity (the kernels loop over the
 // batch's own size, read from P.dyn).  Returns the number of kernels.
-static uint32_t launch_batch(BdptBatcher* b, uint32_t max_depth, cudaStream_t s) {
+static uint32_t launch_batch(BdptBatcher* b, uint32_t max_depth, bool walk, cudaStream_t s) {
     ar_context* ctx = b->ctx;
     const BdParams& P = b->P;
     int* err = ctx->err_flag.as<int>();
@@ -988,7 +1071,11 @@ static uint32_t launch_batch(BdptBatcher* b, uint32_t max_depth, cudaStream_t s)
         KernelScope ks(ctx->prof, s, "bdpt_generate");
         k_bd_generate<<<std::max(1, int(std::min<uint64_t>((2ull * b->batch + 255) / 256, wide))), 256, 0, s>>>(P);
     }
-    for (uint32_t d = 0; d < max_depth; ++d) {
+    if (walk) {
+        KernelScope ks(ctx->prof, s, "bdpt_walk");
+        if (max_depth) k_bd_walk<<<ctx->num_sms * kWalkBlocks, 128, 0, s>>>(P, err);
+    }
+    for (uint32_t d = 0; d < max_depth && !walk; ++d) {
         {
             KernelScope ks(ctx->prof, s, "bdpt_extend");
             k_bd_extend<<<ctx->num_sms * int(ctx->trav_blocks_per_sm), 128, 0, s>>>(P, d, err);
@@ -1017,9 +1104,7 @@ static uint32_t launch_batch(BdptBatcher* b, uint32_t max_depth, cudaStream_t s)
     }
     k_bd_count<<<1, 32, 0, s>>>(P.counts, max_depth, ctx->stats_d.as<unsigned long long>(), err);
     AR_CUDA(cudaGetLastError());
-    // generate, (extend, vertex) per depth, hist/scan/scatter, connect,
-    // shadow, count
-    return 2 * max_depth + 7;
+    return batch_kernels(max_depth, walk);
 }
 
 uint32_t bdpt_run_batch(BdptBatcher* b, const std::vector<BdJob>& jobs, const std::vector<BdSegment>& segs,
@@ -1046,19 +1131,20 @@ uint32_t bdpt_run_batch(BdptBatcher* b, const std::vector<BdJob>& jobs, const st
                             st));
     AR_CUDA(cudaMemcpyAsync(b->dyn_d, b->dyn_h, 2 * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     AR_CUDA(cudaEventRecord(b->staged, st));
-    if (ctx->prof.on) return launch_batch(b, max_depth, st);  // per-stage timing
+    const bool walk = use_walk(nsamples, ctx->num_sms);
+    if (ctx->prof.on) return launch_batch(b, max_depth, walk, st);  // per-stage timing
     if (b->captured_stream != st) {
         for (auto& g : b->graphs)
             if (g) cudaGraphExecDestroy(g);
         for (auto& g : b->graphs) g = nullptr;
         b->captured_stream = st;
     }
-    cudaGraphExec_t& ge = b->graphs[max_depth];
+    cudaGraphExec_t& ge = b->graphs[2 * max_depth + walk];
     if (!ge) {
         cudaGraph_t graph;
         AR_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         try {
-            launch_batch(b, max_depth, st);
+            launch_batch(b, max_depth, walk, st);
         } catch (...) {
             cudaStreamEndCapture(st, &graph);
             throw;
@@ -1069,7 +1155,7 @@ uint32_t bdpt_run_batch(BdptBatcher* b, const std::vector<BdJob>& jobs, const st
         AR_CUDA(e);
     }
     AR_CUDA(cudaGraphLaunch(ge, st));
-    return 2 * max_depth + 7;
+    return batch_kernels(max_depth, walk);
 }
 
 BdJob make_bdpt_job(const ar_scene* sc, const CameraDev& cam, const ar_integrator_cfg& cfg, uint32_t w, uint32_t h,

@@ -147,3 +147,28 @@ def test_rgb8_does_not_depend_on_size_or_alignment(ctx, h, w, tm, gamma):
     np.testing.assert_array_equal(agentray.film_to_rgb8(ctx, shifted, tm, gamma, 1.5, 4.0).cpu().numpy(), want)
     d = np.abs(want.astype(int) - O.film_to_rgb8(hdr, tm, 4.0, gamma, 1.5).astype(int))
     assert d.max() <= 1 and (d > 0).sum() <= max(1, 1e-3 * d.size)
+
+
+@pytest.mark.parametrize("depth", [0, 1, 9])
+def test_bdpt_small_batches_match_large_ones(ctx, depth):
+    # A batch of few samples traces each subpath through all its bounces in one
+    # launch, a large one bounce by bounce: a 4-spp render above the line against
+    # the sum of its four one-sample shards below it (FP64 films), and the number
+    # of rays they trace.
+    from agentray import distributed as D
+    import torch
+    sc, cam = S.room(seed=4, sphere_levels=(3, 3, 2, 2), n_boxes=40)
+    g = agentray.Scene(ctx, sc)
+    line = torch.cuda.get_device_properties(0).multi_processor_count * 5 * 128 * 3 // 2
+    w, h = 331, line // 331 // 2 + 3  # one sample a pixel below the line, four above it
+    assert w * h < line < 4 * w * h
+    bd = agentray.BidirectionalPathTracer(agentray.BdptConfig(spp=4, max_depth=depth, rr_depth=3, seed=12,
+                                                              film_precision=A.FILM_F64))
+    full = bd.render(g, cam, w, h).rgb.astype(np.float64)
+    stats = ctx.render_stats()
+    parts, rays = [], 0
+    for k in range(4):
+        parts.append(D.render_shard(bd, g, cam, w, h, k, k + 1, np.zeros(w * h * 3, np.float32)).astype(np.float64))
+        rays += ctx.render_stats()["extend_rays"]
+    assert rays == stats["extend_rays"]
+    np.testing.assert_allclose(np.sum(parts, axis=0).reshape(h, w, 3), full, rtol=1e-5, atol=1e-6)

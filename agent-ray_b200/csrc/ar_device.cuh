@@ -15,6 +15,7 @@
 #define AR_TRAVERSAL_MIN_BLOCKS 8
 #endif
 #define AR_TRAVERSAL_BOUNDS __launch_bounds__(128, AR_TRAVERSAL_MIN_BLOCKS)
+constexpr int kTraversalThreads = 128;  // threads per block of every kernel that traverses
 // Traversal steps a lane runs between two ray-fetch rounds of its warp: 4 for
 // any hit, whose rays end sooner, 6 for closest hit (1M-triangle soup 19.8 ms at
 // 4, 19.35 at 6, 19.2 at 8; BDPT room's extension 19.0, 19.1, 19.5; shadow rays
@@ -288,10 +289,14 @@ __device__ __forceinline__ uint32_t intersect_node(const WideNode* node, f3 o, f
 //
 // Registers hold only what a node visit and a triangle test read (the current
 // ray, its t limit, the next node, the stack pointer).  What is read once per
-// instance or once per ray lies in named slots below the stack in local
-// memory: the world ray, the best hit so far.  With all of it in scalars the
+// instance or once per ray lies in named slots of cold state: the world ray, the
+// best hit so far.  With all of it in scalars the
 // compiler spilled 120-200 bytes inside the node visit, more local traffic
 // than the stack's; now nothing spills at the 64 registers of 8 blocks per SM.
+// Any hit keeps its cold state in local memory, closest hit (which touches more
+// of it) in shared memory, 80 bytes a thread, whose accesses do not go through to
+// L2: soup 19.4 -> 17.6 ms, BDPT room's extension 18.1 -> 17.7; for any hit that
+// was 0.4-1.8 % slower, the stack in either place costs L1 (7-11 %).
 // 16M rays on the 1M-triangle soup 24.1 -> 20.1 ms, a 139k-triangle scene's
 // extension rays 6.35 -> 5.70 ms and shadow rays 4.11 -> 3.73 ms per
 // 512x512x16 render; 7 blocks (72 registers) 2-12 % slower, 9, 10 and 12
@@ -300,12 +305,15 @@ template <bool kAnyHit>
 struct Traverser {
     static constexpr uint32_t kNodeGroup = 0x80000000u, kMarker = 0x40000000u, kObjectMask = 0x3fffffffu;
     static constexpr uint32_t kInBlas = 8u;  // in `oct`: the current ray is an instance's local ray
-    // slots of the local array: world origin and t_min, world direction and
+    // slots of the cold state: world origin and t_min, world direction and
     // t limit (its best hit), world reciprocals and octant, then the best hit
     // inside the current instance (u, v; slot, scale) and of the ray (u, v;
     // slot, object); the stack proper starts at kStack
     static constexpr int kOxy = 0, kOzT = 1, kDxy = 2, kDzT = 3, kIxy = 4, kIzO = 5, kBestUv = 6, kBest = 7, kHitUv = 8,
-                         kHit = 9, kStack = 10;
+                         kHit = 9, kCold = 10;
+    // where they lie: `cold` + slot * kColdStride; for any hit `cold` is the start of
+    // the local array `mem`, whose stack begins at kStack
+    static constexpr int kColdStride = kAnyHit ? 1 : kTraversalThreads, kStack = kAnyHit ? kCold : 0;
     static constexpr int kSlots = kStack + kTraversalStack;
     const WideNode* geom; // the scene's nodes, triangle and instance records
     f3 o, d, inv;         // the current ray (d is read only inside an instance)
@@ -325,17 +333,17 @@ struct Traverser {
     }
 
     // False when the scene is empty (the ray misses).
-    __device__ __forceinline__ bool start(const DevScene* s, const Ray& r, uint2* mem) {
+    __device__ __forceinline__ bool start(const DevScene* s, const Ray& r, uint2* cold) {
         geom = s->nodes;
         set_ray(r.o, r.d, r.tmin);
         tlim = r.tmax;
-        mem[kOxy] = pk(r.o.x, r.o.y);
-        mem[kOzT] = pk(r.o.z, r.tmin);
-        mem[kDxy] = pk(r.d.x, r.d.y);
-        mem[kDzT] = pk(r.d.z, r.tmax);
-        mem[kIxy] = pk(inv.x, inv.y);
-        mem[kIzO] = make_uint2(__float_as_uint(inv.z), oct);
-        mem[kHit] = make_uint2(kInvalid, kInvalid);
+        cold[kOxy * kColdStride] = pk(r.o.x, r.o.y);
+        cold[kOzT * kColdStride] = pk(r.o.z, r.tmin);
+        cold[kDxy * kColdStride] = pk(r.d.x, r.d.y);
+        cold[kDzT * kColdStride] = pk(r.d.z, r.tmax);
+        cold[kIxy * kColdStride] = pk(inv.x, inv.y);
+        cold[kIzO * kColdStride] = make_uint2(__float_as_uint(inv.z), oct);
+        cold[kHit * kColdStride] = make_uint2(kInvalid, kInvalid);
         node = s->tlas_root;
         sp = 0;
         guard = 0;
@@ -343,16 +351,16 @@ struct Traverser {
     }
 
     // The finished ray's hit (t is the ray's t_max when it missed).
-    __device__ __forceinline__ HitRec result(const uint2* mem) const {
+    __device__ __forceinline__ HitRec result(const uint2* cold) const {
         HitRec h;
         h.t = tlim;
         h.u = h.v = 0.f;
-        h.slot = mem[kHit].x;
+        h.slot = cold[kHit * kColdStride].x;
         h.inst = kInvalid;
         if (!kAnyHit && h.slot != kInvalid) {
-            h.inst = mem[kHit].y;
-            h.u = __uint_as_float(mem[kHitUv].x);
-            h.v = __uint_as_float(mem[kHitUv].y);
+            h.inst = cold[kHit * kColdStride].y;
+            h.u = __uint_as_float(cold[kHitUv * kColdStride].x);
+            h.v = __uint_as_float(cold[kHitUv * kColdStride].y);
         }
         return h;
     }
@@ -372,7 +380,7 @@ struct Traverser {
     // work that leads to the next node to visit, so every active lane of a
     // warp intersects a node in every step.  Returns true when the ray is
     // finished (or failed: *err set).
-    __device__ __forceinline__ bool step(int* err, uint2* mem) {
+    __device__ __forceinline__ bool step(int* err, uint2* mem, uint2* cold) {
         if (++guard > (1u << 22)) { atomicExch(err, 3); return true; }
         uint4 links;  // child_base, tri_base, child_mask, tri_mask
         const uint32_t met = intersect_node(geom + node, o, inv, oct, tmin, tlim, links);
@@ -388,14 +396,14 @@ struct Traverser {
                     float t, u, v;
                     if (tri_test(tr, o, d, tmin, tlim, t, u, v) && t < tlim) {
                         if (kAnyHit) {
-                            if (__fdiv_rn(t, __uint_as_float(mem[kBest].y)) < __uint_as_float(mem[kDzT].y)) {
-                                mem[kHit].x = tr.slot;
+                            if (__fdiv_rn(t, __uint_as_float(cold[kBest * kColdStride].y)) < __uint_as_float(cold[kDzT * kColdStride].y)) {
+                                cold[kHit * kColdStride].x = tr.slot;
                                 return true;
                             }
                         } else {
                             tlim = t;
-                            mem[kBestUv] = pk(u, v);
-                            mem[kBest].x = tr.slot;
+                            cold[kBestUv * kColdStride] = pk(u, v);
+                            cold[kBest * kColdStride].x = tr.slot;
                         }
                     }
                 }
@@ -425,20 +433,20 @@ struct Traverser {
             }
             if (e.y & kMarker) {
                 // Leave the instance: convert the local best back to world t.
-                float best = __uint_as_float(mem[kDzT].y);
+                float best = __uint_as_float(cold[kDzT * kColdStride].y);
                 if (!kAnyHit) {
-                    const uint32_t slot = mem[kBest].x;
+                    const uint32_t slot = cold[kBest * kColdStride].x;
                     if (slot != kInvalid) {
                         const float tw = __fdiv_rn(tlim, __uint_as_float(e.x));
                         if (tw < best) {
                             best = tw;
-                            mem[kHit] = make_uint2(slot, e.y & kObjectMask);
-                            mem[kHitUv] = mem[kBestUv];
+                            cold[kHit * kColdStride] = make_uint2(slot, e.y & kObjectMask);
+                            cold[kHitUv * kColdStride] = cold[kBestUv * kColdStride];
                         }
                     }
                 }
                 tlim = best;
-                const uint2 a = mem[kOxy], b = mem[kOzT], c = mem[kIxy], f = mem[kIzO];
+                const uint2 a = cold[kOxy * kColdStride], b = cold[kOzT * kColdStride], c = cold[kIxy * kColdStride], f = cold[kIzO * kColdStride];
                 o = mk(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(b.x));
                 tmin = __uint_as_float(b.y);
                 inv = mk(__uint_as_float(c.x), __uint_as_float(c.y), __uint_as_float(f.x));
@@ -455,7 +463,7 @@ struct Traverser {
             if (!m3.z) continue;  // mesh without triangles
             const f3 c0 = mk(m0.x, m0.y, m0.z), c1 = mk(m0.w, m1.x, m1.y), c2 = mk(m1.z, m1.w, m2.x),
                      c3 = mk(m2.y, m2.z, m2.w);
-            const uint2 wxy = mem[kDxy], wzt = mem[kDzT];
+            const uint2 wxy = cold[kDxy * kColdStride], wzt = cold[kDzT * kColdStride];
             const float wx = __uint_as_float(wxy.x), wy = __uint_as_float(wxy.y), wz = __uint_as_float(wzt.x);
             // glam transform_point3a / transform_vector3a: ((c0*x + c1*y) + c2*z) + c3
             const f3 ldu = add_rn(add_rn(scale_rn(c0, wx), scale_rn(c1, wy)), scale_rn(c2, wz));
@@ -465,10 +473,10 @@ struct Traverser {
             const f3 lo = add_rn(c3, add_rn(add_rn(scale_rn(c0, o.x), scale_rn(c1, o.y)), scale_rn(c2, o.z)));
             d = normalize_rn(ldu);
             if (kAnyHit) {
-                mem[kBest].y = __float_as_uint(scale);
+                cold[kBest * kColdStride].y = __float_as_uint(scale);
             } else {
-                mem[kBest].x = kInvalid;
-                mem[kDzT].y = __float_as_uint(tlim);
+                cold[kBest * kColdStride].x = kInvalid;
+                cold[kDzT * kColdStride].y = __float_as_uint(tlim);
             }
             tlim = __fmul_rn(tlim, scale);
             set_ray(lo, d, __fmul_rn(tmin, scale));
@@ -479,6 +487,15 @@ struct Traverser {
     }
 };
 
+// Percent of an SM's shared memory that eight blocks' cold state takes, reserve included.
+constexpr int kColdCarveout = 40;
+
+// Declares `cold`, this thread's cold state: in shared memory, or at the start of
+// its local array.
+#define AR_COLD_STATE(any, mem, cold)                                                   \
+    __shared__ uint2 cold_state_[(any) ? 1 : Traverser<any>::kCold * kTraversalThreads]; \
+    uint2* const cold = (any) ? (mem) : cold_state_ + threadIdx.x
+
 // Persistent traversal with dynamic ray fetch.  Every lane of the warp calls
 // this (warp-uniform loop).  `counter` hands out ray indices in [0, n) (reset
 // to 0 before the launch); load(i, scene, ray) fetches ray i and its scene;
@@ -487,6 +504,7 @@ template <bool kAnyHit, class Load, class Store>
 __device__ __forceinline__ void run_traversal(uint32_t* counter, uint32_t n, int* err, Load load, Store store) {
     Traverser<kAnyHit> tr;
     uint2 mem[Traverser<kAnyHit>::kSlots];
+    AR_COLD_STATE(kAnyHit, mem, cold);
     int cur = -1;
     const uint32_t lane = threadIdx.x & 31u;
     // A warp runs every path that any of its rays needs, so few rays are spread
@@ -512,8 +530,8 @@ __device__ __forceinline__ void run_traversal(uint32_t* counter, uint32_t n, int
                     const DevScene* s;
                     Ray r;
                     load(idx, s, r);
-                    if (tr.start(s, r, mem)) cur = int(idx);
-                    else store(idx, tr.result(mem));
+                    if (tr.start(s, r, cold)) cur = int(idx);
+                    else store(idx, tr.result(cold));
                 } else {
                     more = false;
                 }
@@ -523,8 +541,8 @@ __device__ __forceinline__ void run_traversal(uint32_t* counter, uint32_t n, int
         if (cur >= 0) {
 #pragma unroll 1
             for (int k = 0; k < (kAnyHit ? kStepsAny : kStepsClosest); ++k) {
-                if (tr.step(err, mem)) {
-                    store(uint32_t(cur), tr.result(mem));
+                if (tr.step(err, mem, cold)) {
+                    store(uint32_t(cur), tr.result(cold));
                     cur = -1;
                     break;
                 }

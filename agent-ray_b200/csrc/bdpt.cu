@@ -441,6 +441,7 @@ __global__ void __launch_bounds__(128, kWalkBlocks) k_bd_walk(const __grid_const
     const uint32_t n = P.counts[0], lane = threadIdx.x & 31u;
     Traverser<false> tr;
     uint2 mem[Traverser<false>::kSlots];
+    AR_COLD_STATE(false, mem, cold);
     uint32_t q = kInvalid, depth = 0;  // this lane's subpath, kInvalid: none
     f3 ro, rd;
     float tmin = 0.f, tmax = 0.f;
@@ -466,17 +467,17 @@ __global__ void __launch_bounds__(128, kWalkBlocks) k_bd_walk(const __grid_const
         bool busy = false;
         if (q != kInvalid) {
             J = &P.jobs[P.sjob[q >> 1]];
-            busy = tr.start(&J->sc, Ray{ro, rd, tmin, tmax}, mem);
+            busy = tr.start(&J->sc, Ray{ro, rd, tmin, tmax}, cold);
         }
         while (__any_sync(0xffffffffu, busy)) {
             if (busy) {
 #pragma unroll 1
-                for (int k = 0; k < kStepsClosest && busy; ++k) busy = !tr.step(err, mem);
+                for (int k = 0; k < kStepsClosest && busy; ++k) busy = !tr.step(err, mem, cold);
             }
         }
         bool cont = false;
         if (q != kInvalid) {
-            const HitRec h = tr.result(mem);
+            const HitRec h = tr.result(cold);
             f3 no, nd;
             cont = h.slot != kInvalid && bd_vertex(P, *J, q, depth, ro, rd, h.t, h.u, h.v, h.slot, h.inst, no, nd);
             if (cont) {
@@ -992,6 +993,7 @@ BdptBatcher* bdpt_create(ar_context* ctx, uint32_t max_depth_cap, uint32_t batch
     auto b = std::make_unique<BdptBatcher>();
     b->ctx = ctx;
     AR_CUDA(cudaFuncSetAttribute(k_bd_connect, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTileMax)));
+    AR_CUDA(cudaFuncSetAttribute(k_bd_extend, cudaFuncAttributePreferredSharedMemoryCarveout, kColdCarveout));
     b->max_depth_cap = max_depth_cap;
     b->batch = batch;
     b->mem.alloc(bdpt_batch_bytes(max_depth_cap, batch));
@@ -1100,7 +1102,20 @@ static uint32_t launch_batch(BdptBatcher* b, uint32_t max_depth, bool walk, cuda
     }
     {
         KernelScope ks(ctx->prof, s, "bdpt_shadow");
-        k_bd_shadow<<<ctx->num_sms * int(ctx->trav_blocks_per_sm), 128, 0, s>>>(P, err);
+        // A large batch's shadow rays may run beside another lane's extension: with the
+        // same split of L1 an SM takes blocks of both (BDPT room 51.5 -> 50.4 ms, its
+        // shadow stage alone 18.4 -> 19.2; a small batch, alone on the GPU, keeps all of
+        // L1: 309 us against 320).
+        cudaLaunchAttribute split{};
+        split.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        split.val.sharedMemCarveout = kColdCarveout;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(ctx->num_sms * ctx->trav_blocks_per_sm);
+        cfg.blockDim = dim3(kTraversalThreads);
+        cfg.stream = s;
+        cfg.attrs = &split;
+        cfg.numAttrs = walk ? 0 : 1;
+        AR_CUDA(cudaLaunchKernelEx(&cfg, k_bd_shadow, P, err));
     }
     k_bd_count<<<1, 32, 0, s>>>(P.counts, max_depth, ctx->stats_d.as<unsigned long long>(), err);
     AR_CUDA(cudaGetLastError());

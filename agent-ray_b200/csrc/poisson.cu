@@ -26,6 +26,34 @@ namespace ar {
 
 namespace {
 
+// Launches `kernel` so that it is set up while the kernel before it on the stream
+// still drains; it begins with after_previous(), which returns once all earlier
+// work of the stream is complete and visible.  A solve is a chain of short kernels
+// (128 of 5 to 14 us for 64 iterations of conjugate gradient), and launch and ramp-up
+// were up to a third of it.  Unchained -> chained: conjugate gradient to 1e-6, 256^2
+// 919 -> 613 us, 511x513 1191 -> 859, 512^2 1148 -> 831, 1024^2 2124 -> 1810; 200
+// iterations of SOR, 64^2 284 -> 234, 256^2 299 -> 259, 512^2 456 -> 370, 333x701
+// 455 -> 359, 1024^2 1285 -> 1223.  No kernel lets its successor start before it ends: blocks that
+// only wait took room from those that work (a trigger at the start of the conjugate
+// gradient's kernels: 970 us for 512^2 and 2311 for 1024^2; for SOR: 379 and 1223).
+template <class... Params, class... Args>
+inline void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared, cudaStream_t stream,
+                           Args... args) {
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = shared;
+    cfg.stream = stream;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    AR_CUDA(cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
+}
+
+__device__ __forceinline__ void after_previous() { cudaGridDependencySynchronize(); }
+
 __global__ void k_rhs(uint32_t w, uint32_t h, const float* __restrict__ primal, const float* __restrict__ gx,
                       const float* __restrict__ gy, float alpha, bool neg_div, float* __restrict__ rhs,
                       float* __restrict__ img) {
@@ -59,14 +87,14 @@ __global__ void k_rhs(uint32_t w, uint32_t h, const float* __restrict__ primal, 
 // neighbour lane's, and the vertical ones lie in the lane's own rows or, at the
 // strip's edge, in shared memory.
 //
-// 200 iterations, whole-image sweeps against this: 64x64 1.69 -> 0.28 ms,
-// 256x256 1.69 -> 0.31, 512x512 2.51 -> 0.46, 1024x1024 4.17 -> 1.29.
+// 200 iterations, whole-image sweeps against this: 64x64 1.69 -> 0.23 ms,
+// 256x256 1.69 -> 0.26, 512x512 2.51 -> 0.37, 1024x1024 4.17 -> 1.22.
 constexpr int kSorRegion = 64, kSorRows = 4, kSorWarps = kSorRegion / kSorRows;
 // Half sweeps a launch (even, so that each starts with the same colour): as many
-// as leave at most one region per SM, at least 10 (of 6, 8, 10, 12 and 16 the
-// best at 1024x1024: 1.56, 1.50, 1.29, 1.44 and 1.64 ms; at 512x512: 0.73, 0.56,
-// 0.46, 0.67, 0.56, where 10 is the last with one region per SM; at 64x64 0.60,
-// 0.50, 0.44, 0.40, 0.32, fewer launches always winning).
+// as leave at most one region per SM, at least 10.  Measured with 8, 10, 12, 16, 20
+// and 24: 1024x1024 1.37, 1.22, 1.33, 1.59, 2.64, 5.34 ms; 512x512, where 10 is the
+// last with one region per SM, 0.43, 0.37, 0.57, 0.50, 0.84, 1.38; 256x256, where 20
+// is, 0.41, 0.37, 0.32, 0.28, 0.26, 0.43; 64x64 0.38, 0.33, 0.30, 0.26, 0.26, 0.25.
 int sor_halo(uint32_t w, uint32_t h, int num_sms) {
     for (int halo : {24, 20, 16, 12}) {
         const uint32_t inner = uint32_t(kSorRegion - 2 * halo);
@@ -82,6 +110,7 @@ __global__ void __launch_bounds__(kSorWarps * 32, 1) k_sor_sweeps(uint32_t w, ui
                                                                   bool clamp) {
     // the first and last row of every strip: [strip][edge][colour][channel][lane]
     __shared__ float edge[kSorWarps + 2][2][2][3][32];
+    after_previous();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int inner = kSorRegion - 2 * halo;
     const int gx0 = int(blockIdx.x % tiles_x) * inner - halo;  // even: region parity = image parity
@@ -269,15 +298,16 @@ __global__ void k_cg_residual(uint32_t w, uint32_t h, const double* b, const dou
 // kCgSlots places, so that hundreds of blocks do not queue on three addresses.
 // Every float goes through the same operations as before: f64 stencil and
 // sums, f32 vectors.  A solve to 1e-6 (64 iterations): 1024x1024 3.00 -> 2.08
-// ms, 512x512 1.87 -> 1.13, 256x256 1.19 -> 0.92.  Not faster: tiles with a rim in shared memory (2.7
-// ms at 1024x1024: their index arithmetic), loads batched four rows ahead (2.4),
-// four floats a thread with neighbours by shuffle (2.6).
+// ms, 512x512 1.87 -> 1.13, 256x256 1.19 -> 0.92 (chained 1.81, 0.83 and 0.61).  Not
+// faster, unchained: tiles with a rim in shared memory (2.7 ms at 1024x1024: their
+// index arithmetic), loads batched four rows ahead (2.4), four floats a thread with
+// neighbours by shuffle (2.6).
 constexpr uint32_t kCgThreads = 192, kCgInner = 32;  // 64 pixels of a row
 
 // Rows a thread walks: fewer halo rows and prologues the more there are, as
-// long as five blocks an SM are left (16 rows against 8, 4 at 1024x1024: 2.12,
-// 2.34, 2.51 ms; 4 against 8, 16 at 512x512: 1.16, 1.27, 1.73; 2 against 4, 8 at
-// 256x256: 0.87, 0.93, 1.15).
+// long as five blocks an SM are left.  Measured with 1, 2, 4, 8 and 16: 1024x1024
+// 3.90, 2.74, 2.19, 2.03, 1.80 ms; 512x512 1.29, 1.00, 0.82, 1.03, 1.45; 256x256 0.63,
+// 0.56, 0.68, 0.86, 1.44.
 uint32_t cg_rows(uint32_t w, uint32_t h, int num_sms) {
     const uint64_t cols = (3 * uint64_t(w) + kCgThreads - 1) / kCgThreads;
     uint32_t rows = 16;
@@ -350,6 +380,7 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_direction(uint32_t w, uint32_
                                                              double alpha, const double* __restrict__ rr,
                                                              const double* __restrict__ rr_prev, double* pq) {
     __shared__ float coef[3];
+    after_previous();
     double a = 0.0;
     const auto each = [&](uint32_t i, float p, double ap) {
         p_out[i] = p;
@@ -373,6 +404,7 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_update(uint32_t w, uint32_t h
                                                           const double* __restrict__ rr,
                                                           const double* __restrict__ pq, double* rr_new) {
     __shared__ float coef[3];
+    after_previous();
     cg_ratio(rr, pq, coef);
     __syncthreads();
     const float al = coef[threadIdx.x % 3u];
@@ -428,8 +460,8 @@ uint64_t poisson_sor_with_scratch(cudaStream_t stream, int num_sms, const ar_int
     const uint32_t tiles_x = (w + inner - 1) / inner, tiles_y = (h + inner - 1) / inner;
     for (uint64_t l = 0; l < launches; ++l) {
         const int sweeps = int(std::min<uint64_t>(halo, half - l * halo));
-        k_sor_sweeps<<<tiles_x * tiles_y, kSorWarps * 32, 0, stream>>>(w, h, tiles_x, halo, sweeps, rhs, src, dst,
-                                                                       cfg.alpha, cfg.sor_omega, l + 1 == launches);
+        launch_chained(k_sor_sweeps, tiles_x * tiles_y, kSorWarps * 32, 0, stream, w, h, tiles_x, halo, sweeps, rhs,
+                       src, dst, cfg.alpha, cfg.sor_omega, l + 1 == launches);
         std::swap(src, dst);
     }
     AR_CUDA(cudaGetLastError());
@@ -491,9 +523,10 @@ uint64_t poisson_reconstruct(ar_context* ctx, const ar_integrator_cfg& cfg, uint
         if (res <= tol || total >= max_total) break;
         for (uint32_t k = 0; k < kCgInner; ++k) {
             double *rr_k = rr + k * kCgSum, *pq_k = pq + k * kCgSum;
-            k_cg_direction<<<blocks, kCgThreads, 0, st>>>(w, h, rows, r, p[(k + 1) & 1], p[k & 1], alpha, rr_k,
-                                                          k ? rr_k - kCgSum : nullptr, pq_k);
-            k_cg_update<<<blocks, kCgThreads, 0, st>>>(w, h, rows, p[k & 1], d, r, alpha, rr_k, pq_k, rr_k + kCgSum);
+            launch_chained(k_cg_direction, blocks, kCgThreads, 0, st, w, h, rows, r, p[(k + 1) & 1], p[k & 1], alpha,
+                           rr_k, k ? rr_k - kCgSum : nullptr, pq_k);
+            launch_chained(k_cg_update, blocks, kCgThreads, 0, st, w, h, rows, p[k & 1], d, r, alpha, rr_k, pq_k,
+                           rr_k + kCgSum);
         }
         total += kCgInner;
         k_cg_accumulate<<<grid, 256, 0, st>>>(3 * n, x, d);

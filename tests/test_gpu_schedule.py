@@ -104,6 +104,38 @@ def test_sor_regions_are_bit_exact(ctx, h, w, iters):
     np.testing.assert_array_equal(out, ref)
 
 
+def test_chained_sor_under_capture(ctx):
+    # The sweeps are launched as a chain; recorded into a graph and replayed
+    # twice (the second replay starts on the first one's output buffer) they give
+    # the plain call's image, bit for bit.
+    import ctypes as C
+
+    import torch
+    from agentray.scene_data import integrator_cfg
+    h, w = 200, 300
+    torch.manual_seed(5)
+    films = [torch.rand(h, w, 3, device="cuda") for _ in range(3)]
+    cfg = integrator_cfg(A.INTEGRATOR_GDPT, alpha=0.2, poisson_iterations=100, sor_omega=1.6,
+                         poisson_solver=A.POISSON_SOR)
+
+    def solve(out, stream):
+        agentray.check(agentray.lib().ar_poisson_sor_static(
+            C.byref(cfg), w, h, *(f.data_ptr() for f in films), out.data_ptr(), C.c_void_p(stream.cuda_stream)))
+
+    plain, replayed = torch.zeros(h, w, 3, device="cuda"), torch.zeros(h, w, 3, device="cuda")
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    solve(plain, stream)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        solve(replayed, torch.cuda.current_stream())
+    graph.replay()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(plain, replayed)
+
+
 @pytest.mark.parametrize("h,w", [(1, 1), (1, 130), (70, 1), (33, 64), (64, 65), (259, 200)])
 def test_cg_sizes_reach_the_exact_solution(ctx, h, w):
     # Images narrower than a block of columns, ragged last blocks and row runs of

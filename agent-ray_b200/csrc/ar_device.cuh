@@ -290,17 +290,16 @@ __device__ __forceinline__ uint32_t intersect_node(const WideNode* node, f3 o, f
 // Registers hold only what a node visit and a triangle test read (the current
 // ray, its t limit, the next node, the stack pointer).  What is read once per
 // instance or once per ray lies in named slots of cold state: the world ray, the
-// best hit so far.  With all of it in scalars the
-// compiler spilled 120-200 bytes inside the node visit, more local traffic
-// than the stack's; now nothing spills at the 64 registers of 8 blocks per SM.
+// best hit so far.  With all of it in scalars the compiler spilled 120-200 bytes
+// inside the node visit, more local traffic than the stack's; now nothing spills at
+// the 64 registers of 8 blocks per SM: 16M rays on the 1M-triangle soup 24.1 ->
+// 20.1 ms, a 139k-triangle scene's extension rays 6.35 -> 5.70 ms and shadow rays
+// 4.11 -> 3.73 ms per 512x512x16 render; 7 blocks (72 registers) 2-12 % slower, 9,
+// 10 and 12 blocks (56, 48, 40 registers, spilling again) 2-5, 5-25 and 13-40 %.
 // Any hit keeps its cold state in local memory, closest hit (which touches more
 // of it) in shared memory, 80 bytes a thread, whose accesses do not go through to
 // L2: soup 19.4 -> 17.6 ms, BDPT room's extension 18.1 -> 17.7; for any hit that
 // was 0.4-1.8 % slower, the stack in either place costs L1 (7-11 %).
-// 16M rays on the 1M-triangle soup 24.1 -> 20.1 ms, a 139k-triangle scene's
-// extension rays 6.35 -> 5.70 ms and shadow rays 4.11 -> 3.73 ms per
-// 512x512x16 render; 7 blocks (72 registers) 2-12 % slower, 9, 10 and 12
-// blocks (56, 48, 40 registers, spilling again) 2-5, 5-25 and 13-40 %.
 template <bool kAnyHit>
 struct Traverser {
     static constexpr uint32_t kNodeGroup = 0x80000000u, kMarker = 0x40000000u, kObjectMask = 0x3fffffffu;

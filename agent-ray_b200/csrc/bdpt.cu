@@ -8,10 +8,12 @@
 //              both subpaths of every sample trace in one wavefront; each hit
 //              appends a vertex (area-measure pdf_fwd) and retroactively sets
 //              pdf_rev of the previous vertex (:338-559)
-//   connect    one thread per sample enumerates the (s, t) strategies with
-//              s + t <= max_depth + 2, evaluates the unweighted contribution
-//              and the power-heuristic MIS weight (FP64 ratio walk, :594-770)
-//              and emits one shadow ray per candidate (:782-1155)
+//              (small batches: walk, the same for all bounces in one launch)
+//   sort       samples counted and scattered by subpath lengths (S, T)
+//   connect    a block takes a tile of samples into shared memory and shares out
+//              their (s, t) strategies with s + t <= max_depth + 2: unweighted
+//              contribution, power-heuristic MIS weight (FP64 ratios, :594-770),
+//              one shadow ray per candidate (:782-1155)
 //   shadow     any-hit test; visible contributions go to the job's film (s >= 2:
 //              the sample's pixel; s = 1: the projected splat pixel)
 // Vertices are stored SoA by (subpath, depth, sample) so each stage reads

@@ -1,7 +1,8 @@
-"""Scheduling edges of the traversal and of the path engine: ray counts around
-the line below which rays are spread over the grid's warps, and renders whose
-paths all start in the first tick against renders refilled from a small pool.
-Both must give what any other split of the same work gives."""
+"""Scheduling edges of the kernels: ray counts around the line below which rays
+are spread over the grid's warps, renders refilled from a small path pool,
+BDPT tiles and batch forms, regions and row runs of the Poisson solvers, the
+chained SOR under capture, 8-bit output at odd sizes and alignments.  Each must
+give what any other split of the same work gives."""
 import numpy as np
 import pytest
 

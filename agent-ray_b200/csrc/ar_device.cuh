@@ -229,8 +229,12 @@ __device__ __forceinline__ uint32_t to_traversal_order(uint32_t v, uint32_t oct)
 // half the scalar fmaf(byte, a, b) of the same operands (measured against the
 // scalar form: served-scene traversal stages -2%, two children per pair instead
 // of the (x, y) / (near z, far z) pairs used here: -0.3..+0.5%, more spills).
-// A child is missed when far - near is negative (exactly when near > far, the
-// rounded difference of two floats keeps its sign); a funnel shift gathers that
+// A child is missed when far - near is negative: exactly when near > far, since
+// the rounded difference of two floats keeps its sign, but for far = -0 against
+// near = +0, whose difference is -0.  The offsets b are therefore formed as
+// x y + 0, which is never -0, so no plane lies at -0 (a ray that starts on a
+// node's low face and leaves through it, t_min = 0, would lose its hit at t = 0;
+// a multiply-add costs what the multiply did).  A funnel shift gathers that
 // sign bit, two instructions a child where a compare, a byte of leaf data and
 // its shifts took about seven.  The traversal kernels issue on 0.75 of the
 // cycles, so instructions are what counts: 16M rays on the 1M-triangle soup
@@ -246,9 +250,9 @@ __device__ __forceinline__ uint32_t intersect_node(const WideNode* node, f3 o, f
     const float ax = __uint_as_float(ex << 23) * inv.x;
     const float ay = __uint_as_float(ey << 23) * inv.y;
     const float az = __uint_as_float(ez << 23) * inv.z;
-    const float bx = (px - o.x) * inv.x;
-    const float by = (py - o.y) * inv.y;
-    const float bz = (pz - o.z) * inv.z;
+    const float bx = __fmaf_rn(px - o.x, inv.x, 0.0f);
+    const float by = __fmaf_rn(py - o.y, inv.y, 0.0f);
+    const float bz = __fmaf_rn(pz - o.z, inv.z, 0.0f);
     // pairs: (x, y) of the near and of the far planes, and (near z, far z)
     const uint64_t AXY = f2_pack(ax, ay), BXY = f2_pack(bx, by), AZZ = f2_pack(az, az), BZZ = f2_pack(bz, bz);
     const uint64_t UNBIAS = f2_pack(-8388608.0f, -8388608.0f);

@@ -512,15 +512,20 @@ __global__ void __launch_bounds__(128, kWalkBlocks) k_bd_walk(const __grid_const
 // the material already worked out, and the MIS prefix sums.  Threads are
 // (strategy, sample): tile_samples consecutive threads take the same strategy
 // (s, t) of the tile's samples.  4.2M samples of the 195k-triangle room at depth
-// 10: sorted copies 2.4 + connection 14.2 -> 8.4 ms, 65k samples of a small scene
-// at depth 8: 310 -> 138 us.  Other shapes (threads x samples, blocks per SM, room
-// / small): 256x32, 2: 8.7 / 152; 512x32, 2: 9.3 / 157; 256x16, 3: 9.0 / 153;
-// 128x16, 5: 9.3 / 139; 64x8, 11: 11.7 / 188; 32x4, 22: 20.7 / 215.  Listing the
-// candidates that a hemisphere test keeps and evaluating them 32 at a time, as
-// whole warps of mixed strategies, was slower (20.3 / 333).
+// 10: sorted copies 2.4 + connection 14.2 -> 10.5 ms, 65k samples of a small scene
+// at depth 8: 310 -> 178 us.  Rounded like the oracle (see tile_eval); with one
+// reciprocal root for each direction, frame and half vector and one evaluation
+// for value and density it took 8.5 ms and 138 us, but its images left the
+// oracle's by 1e-5 at smooth conductors.  Other shapes in that form (threads x
+// samples, blocks per SM, room / small; this one 8.5 / 138): 256x32, 2: 8.7 / 152;
+// 512x32, 2: 9.3 / 157; 256x16, 3: 9.0 / 153; 128x16, 5: 9.3 / 139; 64x8, 11: 11.7
+// / 188; 32x4, 22: 20.7 / 215.  Out-of-line lobes 11.2 / 189, the local direction's
+// z before its other two components 10.7 / 181.  Listing the candidates that a
+// hemisphere test keeps and evaluating them 32 at a time, as whole warps of mixed
+// strategies, was slower (20.3 / 333).
 enum TileField : uint32_t {
     kFp = 0,      // position
-    kFsmith = 3,  // conductor: sqrt(cos^2 + alpha^2 sin^2) of the direction below
+    kFlambda = 3,  // conductor: ggx_lambda of the direction below
     kFn = 4,      // stored normal
     kFinfo = 7,   // type << 30 | material kind << 28 | material or light index
     kFthr = 8,    // throughput
@@ -581,43 +586,53 @@ struct Tile {
 enum TileInt : uint32_t { kIs, kIt, kIjob, kIpix, kIsample, kIflags };
 constexpr uint32_t kFlagFastMis = 1u, kFlagPointLight = 2u;
 
-// BSDF value and density of a tile vertex toward `wi_world`.  The conductor's
-// masking and shadowing takes the form
-//   D G2 / (4 ci co) = D / (2 (co S(wi) + ci S(wo))),  S(w) = sqrt(c^2 + a^2 (1 - c^2)),
-// equal to ggx_lambda's (1 + L(wi) + L(wo)) with S / c = 1 + 2 L, which needs
-// one root and one division where that form takes two roots and four divisions.
-__device__ __noinline__ float4 glass_eval_pdf(float eta, float alpha, f3 wi, f3 wo) {
+// Value and density of a tile vertex's BSDF: bsdf_eval and bsdf_pdf of the same
+// operands with the same operations, lambda(wo) taken from the tile.  They are
+// not to be rounded otherwise: near h.z = 1 the GGX lobe's h.z^2 (alpha^2 - 1) + 1
+// cancels, so at alpha = 0.1 one rounding of h.z is 1e-5 of the value, and a
+// bright splat carries that into its pixel.  So directions, frames and half
+// vectors keep the square root and the divisions of the inline forms.
+__device__ __noinline__ float4 glass_eval(float eta, float alpha, f3 wi, f3 wo) {
     MatView m{};
-    m.kind = AR_MATERIAL_DIELECTRIC;
     m.alpha = alpha;
     m.eta = eta;
     const f3 f = dielectric_eval(m, wi, wo);
-    return make_float4(f.x, f.y, f.z, dielectric_pdf(m, wi, wo));
+    return make_float4(f.x, f.y, f.z, 0.f);
 }
-__device__ __forceinline__ float smith_root(float alpha, float cos_w) {
-    const float c2 = cos_w * cos_w;
-    return sqrtf(c2 + (alpha * alpha) * (1.0f - c2));
+__device__ __noinline__ float glass_pdf(float eta, float alpha, f3 wi, f3 wo) {
+    MatView m{};
+    m.alpha = alpha;
+    m.eta = eta;
+    return dielectric_pdf(m, wi, wo);
 }
-__device__ __forceinline__ float4 tile_bsdf(const Tile& tl, uint32_t v, f3 wi_world) {
-    const uint32_t kind = (__float_as_uint(tl.at(v, kFinfo)) >> 28) & 3u;
+__device__ __forceinline__ uint32_t tile_kind(const Tile& tl, uint32_t v) {
+    return (__float_as_uint(tl.at(v, kFinfo)) >> 28) & 3u;
+}
+__device__ __forceinline__ f3 tile_eval(const Tile& tl, uint32_t v, f3 wi_world) {
+    const uint32_t kind = tile_kind(tl, v);
     const f3 wi = to_local(tl.frame(v), wi_world), wo = tl.vec(v, kFwo), col = tl.vec(v, kFcol);
-    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (kind == AR_MATERIAL_DIELECTRIC) return glass_eval_pdf(col.x, tl.at(v, kFalpha), wi, wo);
-    if (!same_hemi(wi, wo)) return none;
-    const float ci = fabsf(wi.z), co = fabsf(wo.z);
-    if (kind == AR_MATERIAL_LAMBERTIAN)
-        return make_float4(col.x * kInvPi, col.y * kInvPi, col.z * kInvPi, ci * kInvPi);
-    const f3 hs = wi + wo;
-    const f3 h = hs * __frsqrt_rn(dot(hs, hs));
+    if (kind == AR_MATERIAL_DIELECTRIC) {
+        const float4 f = glass_eval(col.x, tl.at(v, kFalpha), wi, wo);
+        return mk(f.x, f.y, f.z);
+    }
+    if (!same_hemi(wi, wo)) return mk(0.f, 0.f, 0.f);
+    if (kind == AR_MATERIAL_LAMBERTIAN) return col * kInvPi;
+    const float ci = fabsf(wi.z), co = fabsf(wo.z), alpha = tl.at(v, kFalpha);
+    const f3 h = normalize(wi + wo);
+    const f3 f = fresnel_schlick(fabsf(dot(wi, h)), &col.x);
+    const float g = 1.0f / ((1.0f + ggx_lambda(alpha, wi)) + tl.at(v, kFlambda));
+    return f * (ggx_d(alpha, h) * g / ((4.0f * ci) * co));
+}
+__device__ __forceinline__ float tile_pdf(const Tile& tl, uint32_t v, f3 wi_world) {
+    const uint32_t kind = tile_kind(tl, v);
+    const f3 wi = to_local(tl.frame(v), wi_world), wo = tl.vec(v, kFwo);
+    if (kind == AR_MATERIAL_DIELECTRIC) return glass_pdf(tl.at(v, kFcol), tl.at(v, kFalpha), wi, wo);
+    if (!same_hemi(wi, wo)) return 0.f;
+    if (kind == AR_MATERIAL_LAMBERTIAN) return fabsf(wi.z) * kInvPi;
+    const f3 h = normalize(wi + wo);
     const float whwi = fabsf(dot(wi, h));
-    const float c = fminf(fmaxf(1.0f - whwi, 0.0f), 1.0f), c2 = c * c, c5 = c * (c2 * c2);
-    const float alpha = tl.at(v, kFalpha), a2 = alpha * alpha;
-    const float den = (h.z * h.z) * (a2 - 1.0f) + 1.0f;
-    const float pd = (kPi * den) * den;  // D = a2 / pd
-    const float g = a2 / (pd * (2.0f * (co * smith_root(alpha, ci) + ci * tl.at(v, kFsmith))));
-    const float pdf = whwi == 0.f ? 0.f : (a2 * fabsf(h.z)) / (pd * (4.0f * whwi));
-    return make_float4((col.x + (1.0f - col.x) * c5) * g, (col.y + (1.0f - col.y) * c5) * g,
-                       (col.z + (1.0f - col.z) * c5) * g, pdf);
+    if (whwi == 0.f) return 0.f;
+    return ggx_d(tl.at(v, kFalpha), h) * fabsf(h.z) / (4.0f * whwi);
 }
 
 __device__ __forceinline__ float tile_mis(const BdParams& P, const BdJob& J, const Tile& tl, uint32_t s, uint32_t t,
@@ -655,21 +670,15 @@ __device__ __forceinline__ void tile_load(const BdParams& P, const BdJob& J, con
     if (v.type == kTypeSurface) {
         const float4 a = __ldg(P.va + vidx(P, sub, k - 1, si));
         const MatView m = vtx_mat(P, J, v, sub, k, si);
-        // the frame of onb_from_normal
-        Onb o;
-        o.n = v.n * __frsqrt_rn(dot(v.n, v.n));
-        const f3 b = cross(o.n, fabsf(o.n.x) > 0.9f ? mk(0.f, 1.f, 0.f) : mk(1.f, 0.f, 0.f));
-        o.b = b * __frsqrt_rn(dot(b, b));
-        o.t = cross(o.b, o.n);
-        const f3 d = mk(a.x, a.y, a.z) - v.p;
-        const f3 wo = to_local(o, d * __frsqrt_rn(dot(d, d)));
+        const Onb o = onb_from_normal(v.n);
+        const f3 wo = to_local(o, normalize(mk(a.x, a.y, a.z) - v.p));
         tl.put(w, kFon, o.n);
         tl.put(w, kFob, o.b);
         tl.put(w, kFwo, wo);
         const float* c = m.kind == AR_MATERIAL_LAMBERTIAN ? m.albedo : m.f0;
         tl.put(w, kFcol, m.kind == AR_MATERIAL_DIELECTRIC ? mk(m.eta, 0.f, 0.f) : mk(c[0], c[1], c[2]));
         tl.at(w, kFalpha) = m.alpha;
-        tl.at(w, kFsmith) = smith_root(m.alpha, wo.z);
+        tl.at(w, kFlambda) = ggx_lambda(m.alpha, wo);
         info |= m.kind << 28;
     }
     tl.at(w, kFinfo) = __uint_as_float(info);
@@ -677,8 +686,9 @@ __device__ __forceinline__ void tile_load(const BdParams& P, const BdJob& J, con
 
 // connect_bdpt for s >= 2 (:782-1044) + the t == 0 extension.  Emits a shadow
 // ray with the MIS-weighted contribution, or deposits directly when t == 0.
-// One direction serves both ends of a connection: the value, the density and
-// the geometry term of a strategy all take it and the two cosines.
+// The value and the geometry terms of a strategy take one direction, d / |d|,
+// the densities (as in the reference) the other rounding, d * (1 / |d|); both
+// serve either end.
 __device__ __forceinline__ void connect_general(const BdParams& P, const BdJob& J, const Tile& tl, uint32_t s,
                                                 uint32_t t) {
     const uint32_t vz = tl.vertex(0, s - 1);
@@ -700,14 +710,18 @@ __device__ __forceinline__ void connect_general(const BdParams& P, const BdJob& 
     const f3 d = yp - zp;
     const float d2 = dot(d, d);
     if (d2 < 1e-10f) return;
-    const float inv_dist = __frsqrt_rn(d2), inv_d2 = inv_dist * inv_dist;
-    const f3 wi_z = d * inv_dist;
+    const float dist = sqrtf(d2);
+    const f3 wi_z = d / dist;
     const float dz = dot(wi_z, zn), dy = dot(-wi_z, yn);
-    const float4 ez = tile_bsdf(tl, vz, wi_z);
-    const f3 f_z = mk(ez.x, ez.y, ez.z);
+    // the shadow ray
+    const f3 so = zp + (zn * 1e-4f) * signum(dz);
+    const f3 sd = (yp + (yn * 1e-4f) * signum(dy)) - so;
+    const float sdist = length(sd);
+    if (sdist < 1e-6f) return;
+    const f3 f_z = tile_eval(tl, vz, wi_z);
     if (is_zero(f_z)) return;
-    const float cz = fabsf(dz), cy = fabsf(dy);
-    const f3 thr_z = tl.vec(vz, kFthr);
+    const float cz = fabsf(dz), cy = fabsf(dy), g = cz * cy / d2;
+    const f3 wn = d * (1.0f / dist), thr_z = tl.vec(vz, kFthr);
     f3 c;
     float pdf_y;
     if (t == 1) {
@@ -717,27 +731,21 @@ __device__ __forceinline__ void connect_general(const BdParams& P, const BdJob& 
             f3 lwi, lrad;
             float ldist, lpdf;
             if (!light_sample(L, zp, 0.f, 0.f, lwi, ldist, lrad, lpdf)) return;
-            const float4 ed = tile_bsdf(tl, vz, lwi);
-            c = ((thr_z * mk(ed.x, ed.y, ed.z)) * fabsf(dot(zn, lwi))) * lrad;
+            c = ((thr_z * tile_eval(tl, vz, lwi)) * fabsf(dot(zn, lwi))) * lrad;
         } else {
             if (dy <= 0.f) return;
-            c = ((thr_z * f_z) * (cz * cy * inv_d2)) * tl.vec(vy, kFthr);
+            c = ((thr_z * f_z) * g) * tl.vec(vy, kFthr);
         }
-        pdf_y = light_pdf_emission_dir(L, -wi_z);
+        if (max3(c) <= 0.f) return;
+        pdf_y = light_pdf_emission_dir(L, -wn);
     } else {
-        const float4 ey = tile_bsdf(tl, vy, -wi_z);
-        const f3 f_y = mk(ey.x, ey.y, ey.z);
+        const f3 f_y = tile_eval(tl, vy, -wi_z);
         if (is_zero(f_y)) return;
-        c = (((thr_z * f_z) * (cz * cy * inv_d2)) * f_y) * tl.vec(vy, kFthr);
-        pdf_y = ey.w;
+        c = (((thr_z * f_z) * g) * f_y) * tl.vec(vy, kFthr);
+        if (max3(c) <= 0.f) return;
+        pdf_y = tile_pdf(tl, vy, -wn);
     }
-    if (max3(c) <= 0.f) return;
-    // the shadow ray, with the reference's operations
-    const f3 so = zp + (zn * 1e-4f) * signum(dz);
-    const f3 sd = (yp + (yn * 1e-4f) * signum(dy)) - so;
-    const float sdist = length(sd);
-    if (sdist < 1e-6f) return;
-    const float w = tile_mis(P, J, tl, s, t, pdf_y * cz * inv_d2, ez.w * cy * inv_d2);
+    const float w = tile_mis(P, J, tl, s, t, pdf_y * cz / d2, tile_pdf(tl, vz, wn) * cy / d2);
     push_shadow(P, tl.word(kIjob), so, normalize(sd / sdist), sdist * (1.0f - 1e-4f), c * w, tl.word(kIpix));
 }
 
@@ -764,14 +772,13 @@ __device__ __forceinline__ void connect_s1(const BdParams& P, const BdJob& J, co
     if (px < 0.f || px >= float(J.width) || py < 0.f || py >= float(J.height)) return;
     const float c2 = ct * ct, c4 = c2 * c2;
     const float we = 1.0f / (J.cam.area * c4);
-    const float4 ey = tile_bsdf(tl, vy, wi);
-    const f3 f_y = mk(ey.x, ey.y, ey.z);
+    const f3 f_y = tile_eval(tl, vy, wi);
     if (is_zero(f_y)) return;
     const float dy = dot(yn, wi);
     const float gf = fabsf(dy) / (dist * dist);
     const f3 c = ((tl.vec(vy, kFthr) * f_y) * gf) * we;
     if (max3(c) <= 0.f) return;
-    const float pdf_cl = pdf_sa_to_area(ey.w, yp, co, tl.vec(tl.vertex(0, 0), kFn));
+    const float pdf_cl = pdf_sa_to_area(tile_pdf(tl, vy, wi), yp, co, tl.vec(tl.vertex(0, 0), kFn));
     const float w = tile_mis(P, J, tl, 1, t, 0.f, pdf_cl);
     const uint32_t ix = min(uint32_t(px), J.width - 1), iy = min(uint32_t(py), J.height - 1);
     const f3 o = yp + (yn * 1e-4f) * signum(dy);

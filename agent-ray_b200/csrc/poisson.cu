@@ -31,11 +31,16 @@ namespace {
 // work of the stream is complete and visible.  A solve is a chain of short kernels
 // (128 of 5 to 14 us for 64 iterations of conjugate gradient), and launch and ramp-up
 // were up to a third of it.  Unchained -> chained: conjugate gradient to 1e-6, 256^2
-// 919 -> 613 us, 511x513 1191 -> 859, 512^2 1148 -> 831, 1024^2 2124 -> 1810; 200
+// 919 -> 609 us, 511x513 1191 -> 889, 512^2 1148 -> 828, 1024^2 2124 -> 1832; 200
 // iterations of SOR, 64^2 284 -> 234, 256^2 299 -> 259, 512^2 456 -> 370, 333x701
 // 455 -> 359, 1024^2 1285 -> 1223.  No kernel lets its successor start before it ends: blocks that
 // only wait took room from those that work (a trigger at the start of the conjugate
 // gradient's kernels: 970 us for 512^2 and 2311 for 1024^2; for SOR: 379 and 1223).
+// What a chained kernel reads may still be written while it is set up.  So no
+// buffer that it reads is __restrict__: that would allow loads of the read-only
+// path, which hold for data that stays as it is for the kernel's whole life, and
+// loads moved above the wait.  (With the qualifiers conjugate gradient took 1802
+// us for 1024^2 and 817 for 512^2, SOR the same.)
 template <class... Params, class... Args>
 inline void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared, cudaStream_t stream,
                            Args... args) {
@@ -104,8 +109,7 @@ int sor_halo(uint32_t w, uint32_t h, int num_sms) {
 }
 
 __global__ void __launch_bounds__(kSorWarps * 32, 1) k_sor_sweeps(uint32_t w, uint32_t h, uint32_t tiles_x, int halo, int sweeps,
-                                                                  const float* __restrict__ rhs,
-                                                                  const float* __restrict__ in,
+                                                                  const float* rhs, const float* in,
                                                                   float* __restrict__ out, float alpha, float omega,
                                                                   bool clamp) {
     // the first and last row of every strip: [strip][edge][colour][channel][lane]
@@ -375,10 +379,9 @@ __device__ __forceinline__ void cg_walk(uint32_t w, uint32_t h, uint32_t rows, d
 
 // p = r + beta p (beta = rr / rr_prev; the first iteration takes p = r), pq += p.Ap
 __global__ void __launch_bounds__(kCgThreads) k_cg_direction(uint32_t w, uint32_t h, uint32_t rows,
-                                                             const float* __restrict__ r,
-                                                             const float* __restrict__ p_in, float* __restrict__ p_out,
-                                                             double alpha, const double* __restrict__ rr,
-                                                             const double* __restrict__ rr_prev, double* pq) {
+                                                             const float* r, const float* p_in,
+                                                             float* __restrict__ p_out, double alpha,
+                                                             const double* rr, const double* rr_prev, double* pq) {
     __shared__ float coef[3];
     after_previous();
     double a = 0.0;
@@ -399,10 +402,8 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_direction(uint32_t w, uint32_
 
 // d += al p, r -= al (A p), al = rr / pq; rr_new += r.r
 __global__ void __launch_bounds__(kCgThreads) k_cg_update(uint32_t w, uint32_t h, uint32_t rows,
-                                                          const float* __restrict__ p, float* __restrict__ d,
-                                                          float* __restrict__ r, double alpha,
-                                                          const double* __restrict__ rr,
-                                                          const double* __restrict__ pq, double* rr_new) {
+                                                          const float* p, float* d, float* r, double alpha,
+                                                          const double* rr, const double* pq, double* rr_new) {
     __shared__ float coef[3];
     after_previous();
     cg_ratio(rr, pq, coef);

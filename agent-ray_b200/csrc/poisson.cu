@@ -198,6 +198,39 @@ __global__ void __launch_bounds__(kSorWarps * 32, 1) k_sor_sweeps(uint32_t w, ui
         }
 }
 
+// One half sweep over the whole image, in place: the pixels with (x + y) & 1 ==
+// parity.  For images too thin to fill regions (see sor_thin).
+__global__ void k_sor_half(uint32_t w, uint32_t h, uint32_t parity, const float* rhs, float* img, float alpha,
+                           float omega) {
+    after_previous();
+    const uint32_t half_w = (w + 1) / 2;
+    const uint32_t n = half_w * h;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const uint32_t y = k / half_w;
+        const uint32_t x = 2 * (k - y * half_w) + ((y + parity) & 1u);
+        if (x >= w) continue;
+        const uint32_t i = 3 * (y * w + x);
+        const int nn = (x > 0) + (x + 1 < w) + (y > 0) + (y + 1 < h);
+        const float inv = 1.0f / (alpha + float(nn));
+        for (uint32_t c = i; c < i + 3; ++c) {
+            float s = 0.f;
+            if (x > 0) s += img[c - 3];
+            if (x + 1 < w) s += img[c + 3];
+            if (y > 0) s += img[c - 3 * w];
+            if (y + 1 < h) s += img[c + 3 * w];
+            img[c] = (1.0f - omega) * img[c] + omega * ((rhs[c] + s) * inv);
+        }
+    }
+}
+
+// Whether whole-image half sweeps are faster than regions: a region costs 4 to 5 ns
+// a half sweep however few of its pixels lie in the image, a whole-image half sweep
+// 2.2 us + 7.5 ns per 1000 pixels.  200 iterations, height x width, regions / whole
+// image: 1x100000 3670 / 936 us, 1x1000000 35740 / 3452, 8x262144 9758 / 7323; on
+// the other side of the line (whole image unchained) 1x10000 519 / 1686, 8x32768
+// 1476 / 2509, 16x65536 2682 / 4249, 1024x1024 1219 / 4165.
+bool sor_thin(uint64_t regions, uint64_t pixels) { return regions > 500 + pixels / 600; }
+
 __global__ void k_clamp(size_t n, const float* __restrict__ in, float* __restrict__ out) {
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
         out[i] = in[i] > 0.f ? in[i] : 0.f;
@@ -446,19 +479,20 @@ uint64_t poisson_sor_with_scratch(cudaStream_t stream, int num_sms, const ar_int
     // and out so that the last one ends in out
     const int halo = sor_halo(w, h, num_sms);
     const uint64_t half = 2 * uint64_t(cfg.poisson_iterations), launches = (half + halo - 1) / halo;
-    float* src = launches & 1 ? img : out;
-    float* dst = launches & 1 ? out : img;
-    if (launches == 0) {
-        k_rhs<<<grid, 256, 0, stream>>>(w, h, primal, gx, gy, cfg.alpha, neg_div, rhs, img);
-        k_clamp<<<grid, 256, 0, stream>>>(3 * n, img, out);
-        AR_CUDA(cudaGetLastError());
-        return 2;
-    }
-    k_rhs<<<grid, 256, 0, stream>>>(w, h, primal, gx, gy, cfg.alpha, neg_div, rhs, img);
-    if (src != img)
-        AR_CUDA(cudaMemcpyAsync(src, img, 3 * n * sizeof(float), cudaMemcpyDeviceToDevice, stream));
     const uint32_t inner = uint32_t(kSorRegion - 2 * halo);
     const uint32_t tiles_x = (w + inner - 1) / inner, tiles_y = (h + inner - 1) / inner;
+    k_rhs<<<grid, 256, 0, stream>>>(w, h, primal, gx, gy, cfg.alpha, neg_div, rhs, img);
+    if (launches == 0 || sor_thin(uint64_t(tiles_x) * tiles_y, n)) {
+        for (uint64_t k = 0; k < half; ++k)
+            launch_chained(k_sor_half, grid, 256, 0, stream, w, h, uint32_t(k & 1), rhs, img, cfg.alpha, cfg.sor_omega);
+        k_clamp<<<grid, 256, 0, stream>>>(3 * n, img, out);
+        AR_CUDA(cudaGetLastError());
+        return 2 + half;
+    }
+    float* src = launches & 1 ? img : out;
+    float* dst = launches & 1 ? out : img;
+    if (src != img)
+        AR_CUDA(cudaMemcpyAsync(src, img, 3 * n * sizeof(float), cudaMemcpyDeviceToDevice, stream));
     for (uint64_t l = 0; l < launches; ++l) {
         const int sweeps = int(std::min<uint64_t>(halo, half - l * halo));
         launch_chained(k_sor_sweeps, tiles_x * tiles_y, kSorWarps * 32, 0, stream, w, h, tiles_x, halo, sweeps, rhs,

@@ -341,16 +341,35 @@ __global__ void k_cg_residual(uint32_t w, uint32_t h, const double* b, const dou
 // neighbours by shuffle (2.6).
 constexpr uint32_t kCgThreads = 192, kCgInner = 32;  // 64 pixels of a row
 
+// How threads share the floats of an image.
+struct CgShape {
+    uint32_t w, h;   // of the walk
+    uint32_t rows;   // that a thread walks down
+    uint32_t log2p;  // a block is 2^log2p pixels wide and takes 64 >> log2p runs of rows
+};
+
 // Rows a thread walks: fewer halo rows and prologues the more there are, as
 // long as five blocks an SM are left.  Measured with 1, 2, 4, 8 and 16: 1024x1024
 // 3.90, 2.74, 2.19, 2.03, 1.80 ms; 512x512 1.29, 1.00, 0.82, 1.03, 1.45; 256x256 0.63,
 // 0.56, 0.68, 0.86, 1.44.
-uint32_t cg_rows(uint32_t w, uint32_t h, int num_sms) {
-    const uint64_t cols = (3 * uint64_t(w) + kCgThreads - 1) / kCgThreads;
-    uint32_t rows = 16;
-    while (rows > 1 && cols * ((h + rows - 1) / rows) < uint64_t(5 * num_sms)) rows /= 2;
-    while ((h + rows - 1) / rows > 65535u) rows *= 2;  // the grid's y extent
-    return rows;
+// A block takes several runs of a narrow image (of 8 rows up to 16 pixels: 200000x5
+// 2.98 ms, with 16 rows 3.32, with 4 3.30), a thread several columns, the grid's
+// width apart, of a low one, and a column of pixels is walked as the row that it is
+// in memory (the same operations).  Against 64 pixels of one run a block: 1000000x1
+// 38.9 -> 2.55 ms, 500000x2 25.5 -> 2.9, 1x1000000 3.57 -> 2.55, 2000x3 616 -> 480 us.
+CgShape cg_shape(uint32_t w, uint32_t h, int num_sms, dim3& grid) {
+    CgShape s{w == 1 ? h : w, w == 1 ? 1u : h, 16, 6};
+    while (s.log2p > 0 && (1u << (s.log2p - 1)) >= s.w) s.log2p--;
+    if (s.log2p <= 4) s.rows = 8;
+    const uint32_t cols = uint32_t((uint64_t(s.w) + (1u << s.log2p) - 1) >> s.log2p), runs = 64u >> s.log2p;
+    const auto blocks_y = [&] { return ((s.h + s.rows - 1) / s.rows + runs - 1) / runs; };
+    const uint64_t least = uint64_t(5 * num_sms);
+    while (s.rows > 1 && uint64_t(cols) * blocks_y() < least) s.rows /= 2;
+    while (blocks_y() > 65535u) s.rows *= 2;  // the grid's y extent
+    uint32_t per = 1;                         // columns a thread
+    while (per * std::min(s.rows, s.h) < 16 && uint64_t(cols) * blocks_y() / (2 * per) >= least) per *= 2;
+    grid = dim3((cols + per - 1) / per, blocks_y());
+    return s;
 }
 
 // coef[c] = num / den of channel c (0 where den is 0), from the slots of the two
@@ -381,38 +400,39 @@ __device__ __forceinline__ void cg_add(double a, double* sum) {
     }
 }
 
-// Calls each(i, v, A v) for the floats of this thread's column in its rows;
+// Calls each(i, v, A v) for the floats of this thread's columns in its rows;
 // at(i) gives v of float i (f32).
 template <class At, class Each>
-__device__ __forceinline__ void cg_walk(uint32_t w, uint32_t h, uint32_t rows, double alpha, At at, Each each) {
-    const uint32_t f = blockIdx.x * kCgThreads + threadIdx.x, pitch = 3u * w;
-    const uint32_t y0 = blockIdx.y * rows, y1 = min(h, y0 + rows);
-    if (f >= pitch || y0 >= h) return;
-    const bool left = f >= 3u, right = f + 3u < pitch;
-    const int nx = int(left) + int(right);
-    uint32_t i = y0 * pitch + f;
-    float m32 = at(i);
-    double up = y0 > 0 ? double(at(i - pitch)) : 0.0, mid = double(m32);
+__device__ __forceinline__ void cg_walk(const CgShape& g, double alpha, At at, Each each) {
+    const uint32_t run = (threadIdx.x / 3u) >> g.log2p, lanes = 3u << g.log2p, pitch = 3u * g.w;
+    const uint32_t y0 = (blockIdx.y * (64u >> g.log2p) + run) * g.rows, y1 = min(g.h, y0 + g.rows);
+    if (y0 >= g.h) return;
+    for (uint32_t f = blockIdx.x * lanes + (threadIdx.x - run * lanes); f < pitch; f += gridDim.x * lanes) {
+        const bool left = f >= 3u, right = f + 3u < pitch;
+        const int nx = int(left) + int(right);
+        uint32_t i = y0 * pitch + f;
+        float m32 = at(i);
+        double up = y0 > 0 ? double(at(i - pitch)) : 0.0, mid = double(m32);
 #pragma unroll 4
-    for (uint32_t y = y0; y < y1; ++y, i += pitch) {
-        const float d32 = y + 1 < h ? at(i + pitch) : 0.f;
-        const float l32 = left ? at(i - 3u) : 0.f, r32 = right ? at(i + 3u) : 0.f;
-        const double down = double(d32);
-        double s = double(l32);  // left, right, up, down; outside the image 0
-        s += double(r32);
-        s += up;
-        s += down;
-        const double diag = alpha + (nx + int(y > 0) + int(y + 1 < h));
-        each(i, m32, diag * mid - s);
-        up = mid;
-        mid = down;
-        m32 = d32;
+        for (uint32_t y = y0; y < y1; ++y, i += pitch) {
+            const float d32 = y + 1 < g.h ? at(i + pitch) : 0.f;
+            const float l32 = left ? at(i - 3u) : 0.f, r32 = right ? at(i + 3u) : 0.f;
+            const double down = double(d32);
+            double s = double(l32);  // left, right, up, down; outside the image 0
+            s += double(r32);
+            s += up;
+            s += down;
+            const double diag = alpha + (nx + int(y > 0) + int(y + 1 < g.h));
+            each(i, m32, diag * mid - s);
+            up = mid;
+            mid = down;
+            m32 = d32;
+        }
     }
 }
 
 // p = r + beta p (beta = rr / rr_prev; the first iteration takes p = r), pq += p.Ap
-__global__ void __launch_bounds__(kCgThreads) k_cg_direction(uint32_t w, uint32_t h, uint32_t rows,
-                                                             const float* r, const float* p_in,
+__global__ void __launch_bounds__(kCgThreads) k_cg_direction(CgShape g, const float* r, const float* p_in,
                                                              float* __restrict__ p_out, double alpha,
                                                              const double* rr, const double* rr_prev, double* pq) {
     __shared__ float coef[3];
@@ -426,16 +446,15 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_direction(uint32_t w, uint32_
         cg_ratio(rr, rr_prev, coef);
         __syncthreads();
         const float be = coef[threadIdx.x % 3u];
-        cg_walk(w, h, rows, alpha, [&](uint32_t i) { return r[i] + be * p_in[i]; }, each);
+        cg_walk(g, alpha, [&](uint32_t i) { return r[i] + be * p_in[i]; }, each);
     } else {
-        cg_walk(w, h, rows, alpha, [&](uint32_t i) { return r[i]; }, each);
+        cg_walk(g, alpha, [&](uint32_t i) { return r[i]; }, each);
     }
     cg_add(a, pq);
 }
 
 // d += al p, r -= al (A p), al = rr / pq; rr_new += r.r
-__global__ void __launch_bounds__(kCgThreads) k_cg_update(uint32_t w, uint32_t h, uint32_t rows,
-                                                          const float* p, float* d, float* r, double alpha,
+__global__ void __launch_bounds__(kCgThreads) k_cg_update(CgShape g, const float* p, float* d, float* r, double alpha,
                                                           const double* rr, const double* pq, double* rr_new) {
     __shared__ float coef[3];
     after_previous();
@@ -443,7 +462,7 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_update(uint32_t w, uint32_t h
     __syncthreads();
     const float al = coef[threadIdx.x % 3u];
     double a = 0.0;
-    cg_walk(w, h, rows, alpha, [&](uint32_t i) { return p[i]; },
+    cg_walk(g, alpha, [&](uint32_t i) { return p[i]; },
             [&](uint32_t i, float pv, double ap) {
                 d[i] += al * pv;
                 const float rv = r[i] - al * float(ap);
@@ -534,8 +553,8 @@ uint64_t poisson_reconstruct(ar_context* ctx, const ar_integrator_cfg& cfg, uint
     AR_CUDA(cudaMemsetAsync(bb, 0, kCgSum * sizeof(double), st));
     k_cg_setup<<<grid, 256, 0, st>>>(w, h, primal, gx, gy, alpha,
                                      (cfg.gdpt_flags & AR_GDPT_CONSISTENT_DIVERGENCE) != 0, b, x, bb);
-    const uint32_t rows = cg_rows(w, h, ctx->num_sms);
-    const dim3 blocks((3 * w + kCgThreads - 1) / kCgThreads, (h + rows - 1) / rows);
+    dim3 blocks;
+    const CgShape shape = cg_shape(w, h, ctx->num_sms, blocks);
     double hb[2 * kCgSum];
     double res = 0.0;
     uint32_t total = 0;
@@ -558,9 +577,9 @@ uint64_t poisson_reconstruct(ar_context* ctx, const ar_integrator_cfg& cfg, uint
         if (res <= tol || total >= max_total) break;
         for (uint32_t k = 0; k < kCgInner; ++k) {
             double *rr_k = rr + k * kCgSum, *pq_k = pq + k * kCgSum;
-            launch_chained(k_cg_direction, blocks, kCgThreads, 0, st, w, h, rows, r, p[(k + 1) & 1], p[k & 1], alpha,
+            launch_chained(k_cg_direction, blocks, kCgThreads, 0, st, shape, r, p[(k + 1) & 1], p[k & 1], alpha,
                            rr_k, k ? rr_k - kCgSum : nullptr, pq_k);
-            launch_chained(k_cg_update, blocks, kCgThreads, 0, st, w, h, rows, p[k & 1], d, r, alpha, rr_k, pq_k,
+            launch_chained(k_cg_update, blocks, kCgThreads, 0, st, shape, p[k & 1], d, r, alpha, rr_k, pq_k,
                            rr_k + kCgSum);
         }
         total += kCgInner;

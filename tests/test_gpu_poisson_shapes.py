@@ -1,5 +1,4 @@
-"""Poisson solvers over the shapes that choose their launches: thin images, and
-every overlap and run length that the sizes of images lead to."""
+"""Poisson solvers over the shapes that choose their launches: thin images."""
 import numpy as np
 import pytest
 
@@ -28,3 +27,27 @@ def test_sor_of_thin_images_is_bit_exact(ctx, h, w, iters):
     films = _films(h, w)
     out, _ = agentray.poisson_reconstruct(ctx, *films, 0.2, A.POISSON_SOR, iters, 1.6)
     np.testing.assert_array_equal(out, O.poisson_sor_f32(*films, 0.2, iters, 1.6))
+
+
+_CG_THIN = [(1, 150001), (150001, 1), (60011, 2), (40009, 5), (3, 30001), (30001, 17), (2, 3)]
+
+
+@pytest.mark.parametrize("h,w", _CG_THIN)
+def test_cg_of_thin_images_reaches_the_exact_solution(ctx, h, w):
+    # Thin images, whose blocks take several runs and whose threads several columns.
+    # The Neumann stencil is diagonal under the cosine transform, which gives the
+    # exact solution x*; |x - x*| <= |b - A x| / lambda_min with lambda_min = alpha
+    # = 0.2 and |b - A x| <= 1e-6 |b|, plus the f32 output.
+    from scipy.fft import dctn, idctn
+    primal, gx, gy = _films(h, w)
+    out, res = agentray.poisson_reconstruct(ctx, primal, gx, gy, 0.2, A.POISSON_CG, 2000, 1.6, 1e-6)
+    assert 0 <= res <= 1e-6
+    div = gx.astype(np.float64) + gy
+    div[:, 1:] -= gx[:, :-1]
+    div[1:] -= gy[:-1]
+    b = float(np.float32(0.2)) * primal.astype(np.float64) + div
+    ly, lx = (2 - 2 * np.cos(np.pi * np.arange(n) / n) for n in (h, w))
+    spectrum = float(np.float32(0.2)) + ly[:, None, None] + lx[None, :, None]
+    want = np.maximum(idctn(dctn(b, axes=(0, 1), norm="ortho") / spectrum, axes=(0, 1), norm="ortho"), 0)
+    norm = np.linalg.norm(b.reshape(-1, 3), axis=0)
+    assert np.all(np.abs(out - want) <= 5e-6 * norm + 2e-7 * np.abs(want))

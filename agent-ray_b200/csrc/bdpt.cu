@@ -1063,10 +1063,12 @@ void bdpt_destroy(BdptBatcher* b) {
 uint32_t bdpt_batch_capacity(const BdptBatcher* b) { return b->batch; }
 uint32_t bdpt_max_depth_cap(const BdptBatcher* b) { return b->max_depth_cap; }
 
+// Launches of a batch that trace subpath rays.
+static uint32_t extend_launches(uint32_t max_depth, bool walk) { return walk ? std::min(max_depth, 1u) : max_depth; }
 // generate, walk or (extend, vertex) per depth, hist/scan/scatter, connect,
 // shadow, count
 static uint32_t batch_kernels(uint32_t max_depth, bool walk) {
-    return (walk ? (max_depth ? 1 : 0) : 2 * max_depth) + 7;
+    return extend_launches(max_depth, walk) * (walk ? 1 : 2) + 7;
 }
 
 // The stages of one batch whose jobs reach `max_depth` bounces, on stream
@@ -1250,9 +1252,10 @@ void render_bdpt_film(ar_context* ctx, const ar_scene* sc, const CameraDev& cam,
     std::vector<BdJob> jobs{make_bdpt_job(sc, cam, cfg, w, h, film)};
     jobs[0].first_sample = s0;
     jobs[0].samples = s1 - s0;
-    uint64_t batches = 0;
+    uint64_t batches = 0, extends = 0;
     for (uint64_t begin = 0; begin < total; begin += cap, ++batches) {
         const uint32_t n = uint32_t(std::min<uint64_t>(cap, total - begin));
+        extends += extend_launches(cfg.max_depth, use_walk(n, ctx->num_sms));
         if (two_lanes && (batches & 1))
             bdpt_run_batch(ctx->bdpt2, jobs, {BdSegment{0, 0, n, 0, begin}}, ctx->lane_stream);
         else
@@ -1266,7 +1269,7 @@ void render_bdpt_film(ar_context* ctx, const ar_scene* sc, const CameraDev& cam,
                             ctx->stream));
     ctx->stats_pending = true;
     ctx->last_stats.path_samples = total;
-    ctx->last_stats.extend_launches = batches * cfg.max_depth;
+    ctx->last_stats.extend_launches = extends;
     ctx->last_stats.shadow_launches = batches;
 }
 

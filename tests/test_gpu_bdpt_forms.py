@@ -53,3 +53,19 @@ def test_large_batches_match_oracle(ctx, point_light):
     assert abs(img.mean() - ref.mean()) / ref.mean() < 1e-4
     close = np.abs(img - ref) <= 1e-3 * np.maximum(1.0, np.abs(ref))
     assert close.all(axis=2).mean() >= 0.995, close.all(axis=2).mean()
+
+
+@pytest.mark.parametrize("depth", [0, 1, 5])
+def test_extend_launches_are_counted_as_launched(ctx, depth):
+    # A batch of few samples traces all its bounces in one launch, a large one
+    # each in its own.
+    import torch
+    line = torch.cuda.get_device_properties(0).multi_processor_count * 5 * 128 * 3 // 2
+    sc, cam = S.cornell_box(1)
+    g = agentray.Scene(ctx, sc)
+    w, h = 97, line // 97 // 2
+    assert w * h < line < 4 * w * h
+    for spp, launches in ((1, min(depth, 1)), (4, depth)):
+        agentray.BidirectionalPathTracer(agentray.BdptConfig(spp=spp, max_depth=depth, seed=2)).render(g, cam, w, h)
+        stats = ctx.render_stats()
+        assert stats["extend_launches"] == launches and stats["shadow_launches"] == 1, (spp, stats)

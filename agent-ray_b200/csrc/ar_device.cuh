@@ -368,10 +368,11 @@ struct Traverser {
         return h;
     }
 
-    // A record's address from its offset in 16-byte words (tri_base, which
-    // for TLAS nodes names instance records).
-    __device__ __forceinline__ const float4* record(uint32_t off) const {
-        return reinterpret_cast<const float4*>(geom) + off;
+    // The record that a node's tri_base names: its distance from `geom` in
+    // records, triangles for BLAS nodes, instances for TLAS nodes.
+    template <class Record>
+    __device__ __forceinline__ const Record* record(uint32_t k) const {
+        return reinterpret_cast<const Record*>(geom) + k;
     }
     __device__ __forceinline__ bool push(uint2 e, int* err, uint2* mem) {
         if (sp >= kTraversalStack) { atomicExch(err, 1); return false; }
@@ -394,8 +395,7 @@ struct Traverser {
                 while (tbits) {
                     const uint32_t b = __ffs(tbits) - 1;
                     tbits &= tbits - 1;
-                    const TriRecord tr = load_tri(reinterpret_cast<const TriRecord*>(record(links.y)) +
-                                                  __popc(links.w & ((1u << b) - 1u)));
+                    const TriRecord tr = load_tri(record<TriRecord>(links.y + __popc(links.w & ((1u << b) - 1u))));
                     float t, u, v;
                     if (tri_test(tr, o, d, tmin, tlim, t, u, v) && t < tlim) {
                         if (kAnyHit) {
@@ -460,7 +460,8 @@ struct Traverser {
             const uint32_t b = __ffs(e.y & kSlotBits) - 1;
             const uint32_t rest = e.y & ~(1u << b);
             if (rest & kSlotBits) mem[kStack + sp++] = make_uint2(e.x, rest);
-            const float4* ip = record(e.x) + 4u * __popc(e.y & (kSlotBits << 1) & ((1u << b) - 1u));
+            const float4* ip = reinterpret_cast<const float4*>(
+                record<InstanceRecord>(e.x + __popc(e.y & (kSlotBits << 1) & ((1u << b) - 1u))));
             const float4 m0 = __ldg(ip), m1 = __ldg(ip + 1), m2 = __ldg(ip + 2);
             const uint4 m3 = __ldg(reinterpret_cast<const uint4*>(ip + 3));
             if (!m3.z) continue;  // mesh without triangles

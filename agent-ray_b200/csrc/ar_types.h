@@ -10,7 +10,8 @@
 // Child slot s owns bits 4s..4s+3 of the two masks.  child_mask bit 4s: an
 // internal child at child_base + (its rank among the internal children);
 // tri_mask bits 4s..4s+c-1: a leaf of c primitives, the one of mask bit b at
-// tri_base + popc(tri_mask & ((1 << b) - 1)).  Neither: an empty slot.
+// tri_base + popc(tri_mask & ((1 << b) - 1)), counted in triangle (BLAS) or
+// instance (TLAS) records from the first node.  Neither: an empty slot.
 // Slots are assigned by octant (bit k of s set: child lies on the + side of
 // axis k), so traversal visits slot (i ^ ray_octant) for i = 0..7, an
 // approximately front-to-back order with no sorting.

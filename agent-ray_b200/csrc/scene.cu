@@ -224,29 +224,23 @@ void build_scene_accel(ar_scene* s, const ar_accel_opts* o) {
     const uint32_t worst_stack = tlas_depth + max_blas_depth + 4;
     AR_REQUIRE(worst_stack <= uint32_t(kTraversalStack), AR_ERR_UNSUPPORTED,
                "BVH too deep for the traversal stack (" + std::to_string(worst_stack) + " entries)");
-    // One buffer of nodes, then triangles, then instances; the nodes' leaf
-    // links become 16-byte-word offsets into it, so that the traversal follows
-    // every link from one base address it keeps in registers instead of loading
-    // an array's address from the job before each node, triangle and instance
-    // (139k-triangle scene, 512x512x16: 11.15 -> 11.0 ms; 128x128x4: 1.10 ->
-    // 1.07 ms, where the dependent load is on the critical path).
-    const uint64_t tri_word = nodes.size() * (sizeof(WideNode) / 16);
-    const uint64_t inst_word = tri_word + tris.size() * (sizeof(TriRecord) / 16);
-    const uint64_t words = inst_word + inst_rec.size() * (sizeof(InstanceRecord) / 16);
-    AR_REQUIRE(words <= UINT32_MAX, AR_ERR_UNSUPPORTED, "scene geometry too large (link offsets are 32-bit)");
-    for (size_t i = 0; i < nodes.size(); ++i)
-        nodes[i].tri_base = i < blas_nodes ? uint32_t(tri_word + nodes[i].tri_base * (sizeof(TriRecord) / 16))
-                                           : uint32_t(inst_word + nodes[i].tri_base * (sizeof(InstanceRecord) / 16));
-    s->geom.alloc(words * 16);
-    uint4* geom = s->geom.as<uint4>();
-    const auto put = [&](uint64_t word, const void* src, size_t bytes) {
-        if (bytes) AR_CUDA(cudaMemcpy(geom + word, src, bytes, cudaMemcpyHostToDevice));
+    // One buffer of nodes, then triangles, then instances, so that the traversal
+    // follows every link from one base address it keeps in registers instead of
+    // loading an array's address from the job before each node, triangle and
+    // instance (139k-triangle scene, 512x512x16: 11.15 -> 11.0 ms; 128x128x4: 1.10
+    // -> 1.07 ms, where the dependent load is on the critical path).
+    const GeomLayout lay = geom_layout(nodes.size(), tris.size(), inst_rec.size());
+    AR_REQUIRE(lay.fits, AR_ERR_UNSUPPORTED, "scene geometry too large (links are 32-bit)");
+    for (size_t i = 0; i < nodes.size(); ++i) nodes[i].tri_base += i < blas_nodes ? lay.first_tri : lay.first_inst;
+    s->geom.alloc(lay.bytes);
+    const auto put = [&](uint64_t off, const void* src, size_t bytes) {
+        if (bytes) AR_CUDA(cudaMemcpy(s->geom.as<char>() + off, src, bytes, cudaMemcpyHostToDevice));
     };
     put(0, nodes.data(), nodes.size() * sizeof(WideNode));
-    put(tri_word, tris.data(), tris.size() * sizeof(TriRecord));
-    put(inst_word, inst_rec.data(), inst_rec.size() * sizeof(InstanceRecord));
+    put(uint64_t(lay.first_tri) * sizeof(TriRecord), tris.data(), tris.size() * sizeof(TriRecord));
+    put(uint64_t(lay.first_inst) * sizeof(InstanceRecord), inst_rec.data(), inst_rec.size() * sizeof(InstanceRecord));
     s->view.nodes = s->geom.as<WideNode>();
-    s->view.tris = reinterpret_cast<const TriRecord*>(geom + tri_word);
+    s->view.tris = s->geom.as<TriRecord>() + lay.first_tri;
     s->view.tlas_root = tlas_root;
     // the triangles' shading records, gathered on the device from the uploaded arrays
     s->shade.alloc(std::max<size_t>(1, tris.size()) * sizeof(TriShade));

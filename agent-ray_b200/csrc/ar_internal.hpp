@@ -177,16 +177,18 @@ struct ar_scene {
     struct MeshHost {
         std::vector<float> pos;
         std::vector<uint32_t> idx;
-        bool has_normals = false;
+        std::vector<float> nrm, uv;   // empty when absent
+        std::vector<uint32_t> slots;  // one, or one a triangle
         uint32_t ntri = 0;
+        bool shade = false;           // has shading records, at triangle record + shade_off
+        uint32_t shade_off = 0;
     };
     std::vector<MeshHost> meshes;
     std::vector<ar_object_desc> objects;
     std::vector<std::vector<uint32_t>> object_mats;
     std::vector<float> light_power_weights;
     // device data
-    ar::DevBuf geom, shade, objects_d, meshes_d, indices, normals, slots, mat_table, materials, lights,
-        light_cdf, light_pmf, texcoords, texels, textures;
+    ar::DevBuf geom, shade, objects_d, mat_table, materials, lights, light_cdf, light_pmf, texels, textures;
     ar::DevScene view{};
     ar_scene_stats stats{};
     ar_accel_opts accel{};  // options of the last build

@@ -60,7 +60,7 @@ __device__ __forceinline__ Shade make_shade(const DevScene& sc, f3 ro, f3 rd, fl
     const float4* op = reinterpret_cast<const float4*>(sc.objects + inst);
     const float4 o0 = __ldg(op), o1 = __ldg(op + 1), o2 = __ldg(op + 2), o3 = __ldg(op + 3);
     const uint32_t num_mats = __float_as_uint(o2.w), flags = __float_as_uint(o3.x);
-    const float4* sp = reinterpret_cast<const float4*>(sc.shade + slot);
+    const float4* sp = reinterpret_cast<const float4*>(sc.shade + (slot + __float_as_uint(o3.z)));
     f3 nobj;
     if (flags & kMeshNormals) {
         const float4 a = __ldg(sp), b = __ldg(sp + 1);

@@ -62,31 +62,24 @@ struct alignas(16) ObjectRecord {
     float nmat[9];        // normal matrix columns (inverse-transpose of the linear part)
     uint32_t mesh;
     uint32_t mat_offset;  // into material_table
-    uint32_t num_mats;
+    uint32_t num_mats;    // 1: mat0, whatever the triangle's slot
     uint32_t flags;       // kMeshNormals, kMeshUv
-    uint32_t mat0;        // the first material (the material, when there is one)
-    uint32_t pad[2];
+    uint32_t mat0;
+    uint32_t shade_off;   // triangle record -> shading record, modulo 2^32
+    uint32_t pad;
 };
 static_assert(sizeof(ObjectRecord) == 64, "object record is 64 bytes");
 constexpr uint32_t kMeshNormals = 1u, kMeshUv = 2u;
 
 // What shading reads of a triangle beside its TriRecord, gathered when the
 // acceleration structure is built: its vertices' normals and uv and its material
-// slot.
+// slot.  Only meshes that have one of these for the triangle have such records.
 struct alignas(16) TriShade {
     float n[9];     // normals of the three vertices
     uint32_t slot;  // material slot
     float uv[6];
 };
 static_assert(sizeof(TriShade) == 64, "shading record is 64 bytes");
-
-struct alignas(16) MeshRecord {
-    uint32_t idx_offset;   // into indices (3 per triangle, original order)
-    uint32_t nrm_offset;   // into normals (3 floats per vertex), 0xFFFFFFFF when absent
-    uint32_t slot_offset;  // into material_slots
-    uint32_t num_slots;
-    uint32_t uv_offset;    // into texcoords (2 floats per vertex), 0xFFFFFFFF when absent
-};
 
 struct alignas(16) MaterialRecord {
     uint32_t kind;
@@ -118,7 +111,7 @@ struct alignas(16) LightRecord {
 struct DevScene {
     const WideNode* nodes;  // nodes, triangle and instance records in one buffer
     const TriRecord* tris;  // the triangle records of that buffer
-    const TriShade* shade;  // per triangle record
+    const TriShade* shade;  // at triangle record + its object's shade_off
     const ObjectRecord* objects;
     const uint32_t* material_table;
     const MaterialRecord* materials;

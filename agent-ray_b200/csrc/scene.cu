@@ -42,23 +42,69 @@ void upload(DevBuf& d, const std::vector<T>& h) {
     if (!h.empty()) AR_CUDA(cudaMemcpy(d.ptr, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
 }
 
-// TriShade of every triangle record (of its mesh).
-__global__ void k_gather_shade(const TriRecord* tris, uint32_t n, const MeshRecord* meshes, const uint32_t* indices,
-                               const float* normals, const float* texcoords, const uint32_t* slots, TriShade* out) {
+// A mesh's attributes in one array of 32-bit words: indices (3 a triangle, original
+// order), normals (3 a vertex), uv (2 a vertex), material slots.
+struct MeshAttr {
+    static constexpr uint64_t kNone = ~0ull;
+    uint64_t idx = kNone, nrm = kNone, uv = kNone, slots = kNone;  // idx absent: no shading records
+    uint32_t num_slots = 0, shade_off = 0;
+};
+
+// TriShade of the triangle records of meshes that have some.
+__global__ void k_gather_shade(const TriRecord* tris, uint32_t n, const MeshAttr* meshes, const uint32_t* words,
+                               TriShade* out) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t prim = tris[i].prim;
-        const MeshRecord m = meshes[tris[i].mesh];
-        const uint32_t* ix = indices + m.idx_offset + 3 * size_t(prim);
+        const MeshAttr m = meshes[tris[i].mesh];
+        if (m.idx == MeshAttr::kNone) continue;
         TriShade t{};
         for (int k = 0; k < 3; ++k) {
-            if (m.nrm_offset != kInvalid)
-                for (int j = 0; j < 3; ++j) t.n[3 * k + j] = normals[3 * (size_t(m.nrm_offset) + ix[k]) + j];
-            if (m.uv_offset != kInvalid)
-                for (int j = 0; j < 2; ++j) t.uv[2 * k + j] = texcoords[2 * (size_t(m.uv_offset) + ix[k]) + j];
+            const size_t v = words[m.idx + 3 * size_t(prim) + k];
+            if (m.nrm != MeshAttr::kNone)
+                for (int j = 0; j < 3; ++j) t.n[3 * k + j] = __uint_as_float(words[m.nrm + 3 * v + j]);
+            if (m.uv != MeshAttr::kNone)
+                for (int j = 0; j < 2; ++j) t.uv[2 * k + j] = __uint_as_float(words[m.uv + 2 * v + j]);
         }
-        t.slot = m.num_slots == 1 ? slots[m.slot_offset] : slots[m.slot_offset + prim];
-        out[i] = t;
+        t.slot = words[m.slots + (m.num_slots == 1 ? 0 : prim)];
+        out[i + m.shade_off] = t;
     }
+}
+
+// The scene's shading records, gathered on the device from its meshes' attributes,
+// which stay there no longer than that.
+void build_shade(ar_scene* s, const TriRecord* tris, uint32_t n) {
+    std::vector<MeshAttr> meshes(s->meshes.size());
+    std::vector<uint32_t> words;
+    size_t records = 0;
+    const auto add = [&](const auto& v) {
+        const uint64_t at = words.size();
+        words.resize(at + v.size());
+        if (!v.empty()) std::memcpy(words.data() + at, v.data(), v.size() * 4);
+        return at;
+    };
+    for (size_t m = 0; m < meshes.size(); ++m) {
+        const auto& h = s->meshes[m];
+        if (!h.shade) continue;
+        records += h.ntri;
+        meshes[m].idx = add(h.idx);
+        if (!h.nrm.empty()) meshes[m].nrm = add(h.nrm);
+        if (!h.uv.empty()) meshes[m].uv = add(h.uv);
+        meshes[m].slots = add(h.slots);
+        meshes[m].num_slots = uint32_t(h.slots.size());
+        meshes[m].shade_off = h.shade_off;
+    }
+    s->shade.free();
+    s->view.shade = nullptr;
+    if (records == 0) return;
+    s->shade.alloc(records * sizeof(TriShade));
+    s->view.shade = s->shade.as<TriShade>();
+    DevBuf meshes_d, words_d;
+    upload(meshes_d, meshes);
+    upload(words_d, words);
+    k_gather_shade<<<int(std::min<size_t>((size_t(n) + 255) / 256, 4096)), 256>>>(
+        tris, n, meshes_d.as<MeshAttr>(), words_d.as<uint32_t>(), s->shade.as<TriShade>());
+    AR_CUDA(cudaGetLastError());
+    AR_CUDA(cudaStreamSynchronize(nullptr));
 }
 
 struct V3f {
@@ -242,17 +288,7 @@ void build_scene_accel(ar_scene* s, const ar_accel_opts* o) {
     s->view.nodes = s->geom.as<WideNode>();
     s->view.tris = s->geom.as<TriRecord>() + lay.first_tri;
     s->view.tlas_root = tlas_root;
-    // the triangles' shading records, gathered on the device from the uploaded arrays
-    s->shade.alloc(std::max<size_t>(1, tris.size()) * sizeof(TriShade));
-    s->view.shade = s->shade.as<TriShade>();
-    if (!tris.empty()) {
-        const int grid = int(std::min<size_t>((tris.size() + 255) / 256, 4096));
-        k_gather_shade<<<grid, 256>>>(s->view.tris, uint32_t(tris.size()), s->meshes_d.as<MeshRecord>(),
-                                      s->indices.as<uint32_t>(), s->normals.as<float>(), s->texcoords.as<float>(),
-                                      s->slots.as<uint32_t>(), s->shade.as<TriShade>());
-        AR_CUDA(cudaGetLastError());
-        AR_CUDA(cudaStreamSynchronize(nullptr));
-    }
+    build_shade(s, s->view.tris, uint32_t(tris.size()));
     s->stats.num_blas_nodes = blas_nodes;
     s->stats.num_tlas_nodes = tlas_nodes;
     s->stats.num_instances = inst_rec.size();
@@ -273,9 +309,6 @@ void create_scene(ar_context* ctx, const ar_scene_desc* d, ar_scene** out) {
                "at most 2^28 - 1 materials and lights (BDPT vertices pack the index in 28 bits)");
     AR_REQUIRE(d->light_distribution <= AR_LIGHT_DIST_POWER, AR_ERR_INVALID_ARGUMENT, "bad light distribution");
     // meshes
-    std::vector<uint32_t> indices, slots;
-    std::vector<float> normals, texcoords;
-    std::vector<MeshRecord> mrec(d->num_meshes);
     uint64_t ntri_total = 0;
     s->meshes.resize(d->num_meshes);
     for (uint32_t m = 0; m < d->num_meshes; ++m) {
@@ -290,30 +323,24 @@ void create_scene(ar_context* ctx, const ar_scene_desc* d, ar_scene** out) {
             AR_REQUIRE(v < md.num_vertices, AR_ERR_INVALID_ARGUMENT, "mesh " + std::to_string(m) + ": index out of range");
         AR_REQUIRE(md.num_material_slots == 1 || md.num_material_slots == md.num_triangles || md.num_material_slots == 0,
                    AR_ERR_INVALID_ARGUMENT, "material_slots must have 1 or num_triangles entries");
-        mrec[m].idx_offset = uint32_t(indices.size());
-        indices.insert(indices.end(), mh.idx.begin(), mh.idx.end());
-        if (md.normals) {
-            mh.has_normals = true;
-            mrec[m].nrm_offset = uint32_t(normals.size() / 3);
-            normals.insert(normals.end(), md.normals, md.normals + 3 * size_t(md.num_vertices));
-        } else {
-            mrec[m].nrm_offset = kInvalid;
-        }
-        if (md.tex_coords) {
-            mrec[m].uv_offset = uint32_t(texcoords.size() / 2);
-            texcoords.insert(texcoords.end(), md.tex_coords, md.tex_coords + 2 * size_t(md.num_vertices));
-        } else {
-            mrec[m].uv_offset = kInvalid;
-        }
-        mrec[m].slot_offset = uint32_t(slots.size());
-        if (md.num_material_slots == 0 || !md.material_slots) {
-            slots.push_back(0);
-            mrec[m].num_slots = 1;
-        } else {
-            slots.insert(slots.end(), md.material_slots, md.material_slots + md.num_material_slots);
-            mrec[m].num_slots = md.num_material_slots;
-        }
+        if (md.normals) mh.nrm.assign(md.normals, md.normals + 3 * size_t(md.num_vertices));
+        if (md.tex_coords) mh.uv.assign(md.tex_coords, md.tex_coords + 2 * size_t(md.num_vertices));
+        if (md.num_material_slots == 0 || !md.material_slots) mh.slots.assign(1, 0);
+        else mh.slots.assign(md.material_slots, md.material_slots + md.num_material_slots);
+        mh.shade = !mh.nrm.empty() || !mh.uv.empty();
         ntri_total += md.num_triangles;
+    }
+    // a slot a triangle is read by objects of several materials only
+    for (uint32_t i = 0; i < d->num_objects; ++i)
+        if (d->objects[i].mesh < d->num_meshes && d->objects[i].num_materials > 1 &&
+            s->meshes[d->objects[i].mesh].slots.size() > 1)
+            s->meshes[d->objects[i].mesh].shade = true;
+    // triangle records lie mesh after mesh, shading records likewise
+    uint32_t first_tri = 0, first_shade = 0;
+    for (auto& mh : s->meshes) {
+        mh.shade_off = first_shade - first_tri;
+        first_tri += mh.ntri;
+        if (mh.shade) first_shade += mh.ntri;
     }
     // objects
     std::vector<ObjectRecord> orec(d->num_objects);
@@ -337,10 +364,11 @@ void create_scene(ar_context* ctx, const ar_scene_desc* d, ar_scene** out) {
         std::memcpy(orec[i].nmat, nm, sizeof(nm));
         orec[i].mesh = od.mesh;
         orec[i].mat_offset = uint32_t(mat_table.size());
-        orec[i].num_mats = od.num_materials;
-        orec[i].flags = (mrec[od.mesh].nrm_offset != kInvalid ? kMeshNormals : 0u) |
-                        (mrec[od.mesh].uv_offset != kInvalid ? kMeshUv : 0u);
-        orec[i].mat0 = od.materials[0];
+        const auto& mh = s->meshes[od.mesh];
+        orec[i].num_mats = mh.slots.size() > 1 ? od.num_materials : 1;
+        orec[i].flags = (mh.nrm.empty() ? 0u : kMeshNormals) | (mh.uv.empty() ? 0u : kMeshUv);
+        orec[i].mat0 = od.materials[mh.slots.size() > 1 ? 0 : std::min(mh.slots[0], od.num_materials - 1)];
+        orec[i].shade_off = mh.shade_off;
         mat_table.insert(mat_table.end(), od.materials, od.materials + od.num_materials);
     }
     // materials
@@ -428,13 +456,8 @@ void create_scene(ar_context* ctx, const ar_scene_desc* d, ar_scene** out) {
         for (size_t i = 0; i < size_t(td.width) * td.height; ++i)
             texels.push_back(make_float4(lin(td.rgb8[3 * i]), lin(td.rgb8[3 * i + 1]), lin(td.rgb8[3 * i + 2]), 0.f));
     }
-    upload(s->texcoords, texcoords);
     upload(s->texels, texels);
     upload(s->textures, trec);
-    upload(s->indices, indices);
-    upload(s->normals, normals);
-    upload(s->slots, slots);
-    upload(s->meshes_d, mrec);
     upload(s->objects_d, orec);
     upload(s->mat_table, mat_table);
     upload(s->materials, s->materials_h);
@@ -454,9 +477,8 @@ void create_scene(ar_context* ctx, const ar_scene_desc* d, ar_scene** out) {
     s->stats.num_triangles = ntri_total;
     build_scene_accel(s.get(), nullptr);
     size_t bytes = 0;
-    for (DevBuf* b : {&s->geom, &s->shade, &s->objects_d, &s->meshes_d, &s->indices, &s->normals,
-                      &s->slots, &s->mat_table, &s->materials, &s->lights, &s->light_cdf, &s->light_pmf,
-                      &s->texcoords, &s->texels, &s->textures})
+    for (DevBuf* b : {&s->geom, &s->shade, &s->objects_d, &s->mat_table, &s->materials, &s->lights, &s->light_cdf,
+                      &s->light_pmf, &s->texels, &s->textures})
         bytes += b->bytes;
     s->stats.device_bytes = bytes;
     *out = s.release();

@@ -213,6 +213,7 @@ __device__ __noinline__ float mis_weight(const BdParams& P, const BdJob& J, uint
 // r1 = pdf_connect_cam / pdf_fwd(z_{s-1}); the bracket C_s obeys C_1 = 1,
 // C_s = 1 + q_{s-1}^2 C_{s-1}.  The light side is symmetric (D_t), and its
 // t = 1 term counts only for area lights.  Same sums as mis_weight, in FP64.
+// Longer subpaths than kMisCache take mis_weight.
 constexpr uint32_t kMisCache = 16;
 
 __device__ __forceinline__ void film_add(const BdJob& J, uint32_t pix, f3 v) {
@@ -544,8 +545,13 @@ constexpr uint32_t kTileInts = 6;  // per sample: S, T, job, pixel, sample, flag
 constexpr size_t tile_bytes(uint32_t maxv, uint32_t samples) {
     return size_t(samples) * (2 * size_t(maxv) * (kTileFields * 4 + 16) + kTileInts * 4);
 }
-// Samples of a tile: as many as let two blocks share an SM's 227 KB: 32 up to
-// depth 10, 16 up to 21, 8 up to 43, 4 up to 62.
+// Samples of a tile: as many as leave two blocks of an SM a third of its 228 KB as
+// L1: 32 up to depth 10, 16 up to 21, 8 up to 43, 4 up to 62.  Subpaths of more
+// than kMisCache vertices walk their MIS weights in global memory, and with tiles
+// of up to 95,000 bytes that walk missed L1 (room, full-length subpaths: depth 23
+// 4.95 -> 5.38 ms, 25 6.63 -> 8.66, 50 5.23 -> 7.39; up to 113,000: 29 6.96 -> 9.59).
+// Depths 11 and 12, where nothing walks, would gain by 32 samples (1.70 -> 1.51 and
+// 1.81 -> 1.60), 13 not (1.84 -> 1.83), 14 lose (1.87 -> 1.97).
 constexpr size_t kTileMax = 80000;
 constexpr uint32_t tile_samples(uint32_t maxv) {
     uint32_t n = 32;

@@ -75,7 +75,10 @@ __global__ void k_gather_shade(const TriRecord* tris, uint32_t n, const MeshAttr
 void build_shade(ar_scene* s, const TriRecord* tris, uint32_t n) {
     std::vector<MeshAttr> meshes(s->meshes.size());
     std::vector<uint32_t> words;
-    size_t records = 0;
+    size_t records = 0, total = 0;
+    for (const auto& h : s->meshes)
+        if (h.shade) total += h.idx.size() + h.nrm.size() + h.uv.size() + h.slots.size();
+    words.reserve(total);
     const auto add = [&](const auto& v) {
         const uint64_t at = words.size();
         words.resize(at + v.size());

@@ -127,13 +127,30 @@ class Context:
             pass
 
 
+class _SceneHandle(C.c_void_p):
+    """An ar_scene, destroyed with the last reference to its handle (or by
+    close()): `Scene(ctx, data).handle` as an argument of a call keeps the scene
+    for that call although nothing else refers to it."""
+
+    def destroy(self):
+        if self.value:
+            scene, self.value = C.c_void_p(self.value), None
+            lib().ar_scene_destroy(scene)
+
+    def __del__(self):
+        try:
+            self.destroy()
+        except Exception:
+            pass
+
+
 class Scene:
     """Device-resident scene with its acceleration structures (Scene::new)."""
 
     def __init__(self, ctx: Context, data: SceneData):
         self.ctx = ctx
         self.data = data
-        self.handle = C.c_void_p()
+        self.handle = _SceneHandle()
         desc, keep = data.desc()
         check(lib().ar_scene_create(ctx.handle, C.byref(desc), C.byref(self.handle)))
         del keep
@@ -218,15 +235,7 @@ class Scene:
         return occ
 
     def close(self):
-        if self.handle:
-            lib().ar_scene_destroy(self.handle)
-            self.handle = C.c_void_p()
-
-    def __del__(self):
-        try:
-            self.close()
-        except Exception:
-            pass
+        self.handle.destroy()
 
 
 class Film:

@@ -23,7 +23,7 @@ struct alignas(16) BdJob {
 
 // Batch samples [offset, offset + nsamples) are samples
 // [sample_begin, sample_begin + nsamples) of job `job` (index into the
-// batch's job list), number g being pixel g / samples, sample g % samples.
+// batch's job list), numbered as pixel_sample says.
 // Segments are sorted by offset and contiguous.
 struct BdSegment {
     uint32_t job, offset, nsamples, pad;

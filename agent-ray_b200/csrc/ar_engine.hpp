@@ -37,7 +37,7 @@ struct alignas(16) JobDev {
     float inv_spp;
     uint32_t first_sample;
     void* film[3];
-    unsigned long long total_samples;  // W*H*samples; number g is pixel g / samples, sample g % samples
+    unsigned long long total_samples;  // W*H*samples, numbered as pixel_sample says
     unsigned long long next_sample;    // generation cursor (advanced by the plan kernel)
     unsigned long long total_paths;    // samples * roles
     unsigned long long done_paths;     // finished (deposited) paths

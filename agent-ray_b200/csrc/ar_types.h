@@ -127,6 +127,34 @@ struct DevScene {
 };
 
 constexpr uint32_t kInvalid = 0xFFFFFFFFu;
+
+// Pixel and sample of sample number g of an image of npix pixels: runs of samples
+// of one pixel, pixels row by row, run after run of the whole image.  A run keeps a
+// warp's camera rays and what they first hit together (16 samples, against one of
+// every pixel after the other: extension -7%, render -4.5% at 512x512x16 on 139k
+// triangles; 32x32 blocks of pixels in Z order instead of rows gave 0.2% more, 8x4
+// tiles of one sample each 1.4%).  It ends after 64, since samples that finish
+// together add to one pixel one after the other: without an end 64x64x1024 of a
+// small scene at depth 1 took 1.21 ms (one sample of every pixel after the other
+// 1.02, runs of 64 0.86), 512x512x64 of 139k triangles 36.9 (49.0, 36.9; runs of 32
+// 37.1, of 8 37.7).  Up to 1024 pixels, few enough to stay together anyway, 4 are
+// faster: 16x16x4096 at depth 1 0.94 ms without an end (0.51; runs of 64 0.73, of 4
+// 0.47), 4x4x65536 3.08 (1.74; 2.64, 1.74).
+struct PixelSample {
+    uint32_t pixel, sample;
+};
+AR_HD inline PixelSample pixel_sample(unsigned long long g, uint32_t npix, uint32_t samples) {
+    const uint32_t most = npix > 1024u ? 64u : 4u;
+    uint32_t first = 0, run = samples;
+    if (samples > most) {
+        const unsigned long long pass = (unsigned long long)npix * most, k = g / pass;
+        g -= k * pass;
+        first = uint32_t(k) * most;
+        run = samples - first < most ? samples - first : most;
+    }
+    const uint32_t pixel = uint32_t(g / run);
+    return {pixel, first + uint32_t(g % run)};
+}
 constexpr int kTraversalStack = 32;
 
 }  // namespace ar

@@ -268,8 +268,8 @@ __global__ void __launch_bounds__(256) k_bd_generate(BdParams P) {
             const BdSegment sg = P.seg[lo];
             const BdJob& J = P.jobs[sg.job];
             const unsigned long long g = sg.sample_begin + (si - sg.offset);
-            // all samples of a pixel together, as the path engine generates them
-            const uint32_t pixel = uint32_t(g / J.samples), sample = J.first_sample + uint32_t(g % J.samples);
+            const PixelSample ps = pixel_sample(g, J.width * J.height, J.samples);
+            const uint32_t pixel = ps.pixel, sample = J.first_sample + ps.sample;
             const uint64_t key = counter_key(J.seed, pixel, sample);
             if (sub == 0) {
                 P.sjob[si] = sg.job;

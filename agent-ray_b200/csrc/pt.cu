@@ -176,12 +176,8 @@ __global__ void __launch_bounds__(256) k_generate(EngineDev E, int q) {
         const uint32_t rel = k - sg.path_offset;
         const uint32_t si = rel / sg.roles, role = rel - si * sg.roles;
         const unsigned long long g = sg.sample_begin + si;
-        // all samples of a pixel together, pixels row by row: a warp's camera rays
-        // and what they first hit stay together (against one sample of every pixel
-        // after the other: extension -7%, render -4.5% at 512x512x16 on 139k
-        // triangles; 32x32 blocks in Z order instead of rows gave 0.2% more, 8x4
-        // tiles of one sample each 1.4%)
-        const uint32_t pixel = uint32_t(g / J.samples), sample = J.first_sample + uint32_t(g % J.samples);
+        const PixelSample ps = pixel_sample(g, J.width * J.height, J.samples);
+        const uint32_t pixel = ps.pixel, sample = J.first_sample + ps.sample;
         const uint32_t px = pixel % J.width, py = pixel / J.width;
         const bool skip = (role == kRoleRight && px + 1 >= J.width) || (role == kRoleDown && py + 1 >= J.height);
         if (skip) {

@@ -546,19 +546,26 @@ constexpr size_t tile_bytes(uint32_t maxv, uint32_t samples) {
     return size_t(samples) * (2 * size_t(maxv) * (kTileFields * 4 + 16) + kTileInts * 4);
 }
 // Samples of a tile: as many as leave two blocks of an SM a third of its 228 KB as
-// L1: 32 up to depth 10, 16 up to 21, 8 up to 43, 4 up to 62.  Subpaths of more
-// than kMisCache vertices walk their MIS weights in global memory, and with tiles
-// of up to 95,000 bytes that walk missed L1 (room, full-length subpaths: depth 23
-// 4.95 -> 5.38 ms, 25 6.63 -> 8.66, 50 5.23 -> 7.39; up to 113,000: 29 6.96 -> 9.59).
-// Depths 11 and 12, where nothing walks, would gain by 32 samples (1.70 -> 1.51 and
-// 1.81 -> 1.60), 13 not (1.84 -> 1.83), 14 lose (1.87 -> 1.97).
+// L1: 128 up to depth 1, 64 up to 4, 32 up to 10, 16 up to 21, 8 up to 43, 4 up to
+// 62.  What a tile costs beside its strategies (a chain of loads to its vertices,
+// four barriers) weighs the more the fewer strategies there are: 2.1M samples of a
+// small scene, a thread per sample / tiles of 32 / 64 / 128: depth 0 229 / 670 / 376
+// / 224 us, 1 638 / 1304 / 812 / 514, 2 1275 / 1696 / 1045, 4 2434 / 2307 / 1795.
+// Subpaths of more than kMisCache vertices walk their MIS weights in global memory,
+// and with tiles of up to 95,000 bytes that walk missed L1 (room, full-length
+// subpaths: depth 23 4.95 -> 5.38 ms, 25 6.63 -> 8.66, 50 5.23 -> 7.39; up to
+// 113,000: 29 6.96 -> 9.59).  With more than 80,000 depth 2 would gain by 128 samples
+// (1045 -> 867 us), 5 by 64 (2.41 -> 2.03 ms), 11 and 12 by 32 (1.70 -> 1.51 and 1.81
+// -> 1.60), 13 not (1.84 -> 1.83), 14 lose (1.87 -> 1.97).
 constexpr size_t kTileMax = 80000;
+constexpr uint32_t kTileWide = 128;  // at least two rows of threads a tile: the prefix sums take one a side
 constexpr uint32_t tile_samples(uint32_t maxv) {
-    uint32_t n = 32;
+    uint32_t n = kTileWide;
     while (n > 4 && tile_bytes(maxv, n) > kTileMax) n >>= 1;
     return n;
 }
-static_assert(tile_bytes(63, 4) <= kTileMax && kConnectThreads % 32 == 0, "every depth has a tile");
+static_assert(tile_bytes(63, 4) <= kTileMax && kConnectThreads % kTileWide == 0 && kConnectThreads >= 2 * kTileWide,
+              "every depth has a tile");
 
 struct Tile {
     double* pre;  // [vertex][sample]: C_s, D_t
@@ -899,7 +906,7 @@ __global__ void __launch_bounds__(kConnectThreads, kConnectBlocks) k_bd_connect(
                 x = c;
             }
         }
-        // the tile's longest subpaths bound the strategy loop of all its rows
+        // the longest subpaths of a warp's samples bound its strategy loop
         uint32_t sm = S, tm = T;
         for (uint32_t o = 16; o > 0; o >>= 1) {
             sm = max(sm, __shfl_xor_sync(0xffffffffu, sm, o));

@@ -69,3 +69,17 @@ def test_extend_launches_are_counted_as_launched(ctx, depth):
         agentray.BidirectionalPathTracer(agentray.BdptConfig(spp=spp, max_depth=depth, seed=2)).render(g, cam, w, h)
         stats = ctx.render_stats()
         assert stats["extend_launches"] == launches and stats["shadow_launches"] == 1, (spp, stats)
+
+
+@pytest.mark.parametrize("depth,w,h,spp", [(0, 127, 1, 1), (1, 43, 3, 1), (1, 301, 211, 3), (2, 65, 1, 1),
+                                           (3, 97, 5, 2), (4, 301, 211, 3), (5, 33, 31, 1)])
+def test_tiles_of_every_width_match_oracle(ctx, depth, w, h, spp):
+    # The connection's tiles hold the more samples the shallower the render: 128
+    # up to depth 1, 64 up to 4, 32 from 5, the last one ragged, in both forms of
+    # the batch.  Image tests' bars, of the pixels that see anything.
+    sc, cam = S.cornell_box(2, glass=True, textured=True)
+    img, ref = _render(ctx, sc, cam, w, h, spp=spp, max_depth=depth, rr_depth=3, seed=4)
+    assert (w * h * spp) % 32 and np.isfinite(img).all()
+    assert abs(img.sum() - ref.sum()) <= 1e-4 * ref.sum()
+    close = np.abs(img - ref) <= 1e-3 * np.maximum(1.0, np.abs(ref))
+    assert close.all(axis=2).mean() >= 0.995, close.all(axis=2).mean()

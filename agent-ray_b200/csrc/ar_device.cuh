@@ -306,12 +306,13 @@ __device__ __forceinline__ uint32_t intersect_node(const WideNode* node, f3 o, f
 // was 0.4-1.8 % slower, the stack in either place costs L1 (7-11 %).
 template <bool kAnyHit>
 struct Traverser {
-    static constexpr uint32_t kNodeGroup = 0x80000000u, kMarker = 0x40000000u, kObjectMask = 0x3fffffffu;
+    static constexpr uint32_t kNodeGroup = 0x80000000u, kMarker = 0x40000000u;
     static constexpr uint32_t kInBlas = 8u;  // in `oct`: the current ray is an instance's local ray
     // slots of the cold state: world origin and t_min, world direction and
     // t limit (its best hit), world reciprocals and octant, then the best hit
-    // inside the current instance (u, v; slot, scale) and of the ray (u, v;
-    // slot, object); the stack proper starts at kStack
+    // inside the current instance (u, v; slot, the instance's object, for any hit
+    // its scale) and of the ray (u, v; slot, object, all 32 bits of it, which a stack
+    // entry has no room for); the stack proper starts at kStack
     static constexpr int kOxy = 0, kOzT = 1, kDxy = 2, kDzT = 3, kIxy = 4, kIzO = 5, kBestUv = 6, kBest = 7, kHitUv = 8,
                          kHit = 9, kCold = 10;
     // where they lie: `cold` + slot * kColdStride; for any hit `cold` is the start of
@@ -438,12 +439,12 @@ struct Traverser {
                 // Leave the instance: convert the local best back to world t.
                 float best = __uint_as_float(cold[kDzT * kColdStride].y);
                 if (!kAnyHit) {
-                    const uint32_t slot = cold[kBest * kColdStride].x;
-                    if (slot != kInvalid) {
+                    const uint2 hit = cold[kBest * kColdStride];
+                    if (hit.x != kInvalid) {
                         const float tw = __fdiv_rn(tlim, __uint_as_float(e.x));
                         if (tw < best) {
                             best = tw;
-                            cold[kHit * kColdStride] = make_uint2(slot, e.y & kObjectMask);
+                            cold[kHit * kColdStride] = hit;
                             cold[kHitUv * kColdStride] = cold[kBestUv * kColdStride];
                         }
                     }
@@ -473,13 +474,13 @@ struct Traverser {
             const f3 ldu = add_rn(add_rn(scale_rn(c0, wx), scale_rn(c1, wy)), scale_rn(c2, wz));
             const float scale = __fsqrt_rn(dot_rn(ldu, ldu));
             if (scale < FLT_EPSILON) continue;
-            if (!push(make_uint2(__float_as_uint(scale), kMarker | m3.y), err, mem)) return true;
+            if (!push(make_uint2(__float_as_uint(scale), kMarker), err, mem)) return true;
             const f3 lo = add_rn(c3, add_rn(add_rn(scale_rn(c0, o.x), scale_rn(c1, o.y)), scale_rn(c2, o.z)));
             d = normalize_rn(ldu);
             if (kAnyHit) {
                 cold[kBest * kColdStride].y = __float_as_uint(scale);
             } else {
-                cold[kBest * kColdStride].x = kInvalid;
+                cold[kBest * kColdStride] = make_uint2(kInvalid, m3.y);
                 cold[kDzT * kColdStride].y = __float_as_uint(tlim);
             }
             tlim = __fmul_rn(tlim, scale);

@@ -1,6 +1,7 @@
 """Layout of the scene's geometry buffer, compiled for the host: sections that
 do not overlap, and links that reach what a GPU's memory holds."""
 import os
+import re
 import subprocess
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -43,3 +44,14 @@ def test_sections_are_disjoint_and_reach_the_memory(tmp_path):
         assert tri_at + tris * 48 <= inst_at < tri_at + tris * 48 + 64
         assert total == inst_at + inst * 64
     assert [f[3] for f in _layouts(tmp_path, [(1, 1 << 32, 1), (1 << 32, 1, 1), (1, 1, 1 << 32)])] == [0, 0, 0]
+
+
+def test_hits_name_any_object_of_32_bits():
+    # 2^30 objects and more fit the memory, and a stack entry's top bits say what
+    # it is: an object index travels outside the stack.
+    text = open(os.path.join(ROOT, "agent-ray_b200", "csrc", "ar_device.cuh")).read()
+    body = re.sub(r"//[^\n]*", "", text[text.index("struct Traverser {"):text.index("kColdCarveout")])
+    index = "m3.y"  # of the instance record being entered
+    uses = [line.strip() for line in body.splitlines() if index in line]
+    assert uses and not any("push" in u or "kMarker" in u for u in uses), uses
+    assert not re.search(r"& *k\w*Mask", body)
